@@ -37,17 +37,17 @@ template <int P>
 struct AccIO {
     const float *xl;        // feature 0 of the current tile, at this lane's first point
     uint32_t stride;        // floats between features
-    const float *consts;
-    float *stk[N_STACKS];   // per-type stacks, block (slot*W + c), at this lane's first value
+    uint32_t consts;        // shared-memory address of the program's constants
+    uint32_t stk[N_STACKS]; // per-type stacks (shared-memory addresses), block (slot*W + c), at this lane's first value
     __device__ __forceinline__ Vf<P> X(uint32_t f) const { return load_lane<P>(xl + (size_t)f * stride); }
-    __device__ __forceinline__ Vf<P> C(uint32_t i) const { return splat<P>(consts[i]); }
+    __device__ __forceinline__ Vf<P> C(uint32_t i) const { return splat<P>(lds_f32(consts + 4u * i)); }
     template <int W>
     __device__ __forceinline__ Vf<P> S(int t, uint32_t slot, int c) const {
-        return lds_lane<P>(stk[t] + (slot * W + c) * 32u * P);
+        return lds_lane<P>(stk[t] + (slot * W + c) * 128u * P);
     }
     template <int W>
     __device__ __forceinline__ void put(int t, uint32_t slot, int c, const Vf<P> &v) const {
-        sts_lane<P>(stk[t] + (slot * W + c) * 32u * P, v);
+        sts_lane<P>(stk[t] + (slot * W + c) * 128u * P, v);
     }
 };
 

@@ -21,8 +21,11 @@ LIB = PKG / "librsrgpu.so"
 
 SOURCES = ["runtime.cu", "kernels_plain.cu", "kernels_reg.cu", "kernels_grad.cu", "kernels_adj.cu", "encoder.cpp",
            "serving.cu", "lbfgs.cu", "nelder_mead.cu", "cma_es.cu", "ingest.cu", "noalloc.cu"]
+# --jump-table-density: nvcc's default (101) never builds a jump table, and a
+# switch over the ~60 micro-op kinds of a kernel profile then is a tree of
+# compares and branches, 6 levels of it before every micro-op.
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-fmad=false",
-              "-prec-div=true", "-prec-sqrt=true", "-Xcompiler", "-fPIC,-fvisibility=hidden,-ffp-contract=off",
+              "--jump-table-density=1", "-prec-div=true", "-prec-sqrt=true", "-Xcompiler", "-fPIC,-fvisibility=hidden,-ffp-contract=off",
               "-I", str(ROOT / "include"), "-I", str(HERE)]
 
 

@@ -34,6 +34,9 @@
 namespace rsr {
 
 constexpr uint32_t kAdjParams = 32;
+// Words of staged code beside the program's own: a stop entry (two words)
+// behind each sweep, and the entry read (not run) past the last one.
+constexpr uint32_t kAdjStopWords = 6;
 
 // The tape lives in tensor memory (tmem.cuh): one block per SM allocates
 // all 512 columns of its SM's 128 lanes; warp w owns lanes 32 (w % 4) ..
@@ -48,11 +51,8 @@ constexpr uint32_t kAdjParams = 32;
 // lane's gradient sums.
 template <int P>
 struct RevIO : AccIO<P> {
-    // adjoint stacks in the interleaved lane layout (blocks of 32*P floats),
-    // at this lane's first value
-    float *gstk[N_STACKS];  // adjoint stacks, block (slot*W + c)
     uint32_t tm;            // tensor-memory tape: this warp's lanes, column 0
-    float *gacc;            // this lane's f32 gradient sums: gacc[k*32]
+    uint32_t gacc;          // shared-memory address of this lane's f32 gradient sums, one row of 32 a parameter
     uint32_t valid;         // bit q: value q of the lane is a counted point
     // a tape reference (uops.h, kTapeRefX): a tape slot, or the feature or
     // constant the forward value was loaded from
@@ -64,13 +64,17 @@ struct RevIO : AccIO<P> {
     __device__ __forceinline__ void put_tape(uint32_t slot, const Vf<P> &v) const {
         tm_st<P>(tm + slot * (uint32_t)P, v);
     }
+    // A spilled value's adjoint takes the value's own stack slot: the one
+    // micro-op that pops the value reads it into registers (in both sweeps)
+    // before its reverse writes the adjoint, and no later reverse step reads
+    // the forward value (every PUSH has its own slot).
     template <int W>
     __device__ __forceinline__ Vf<P> GS(int t, uint32_t slot, int c) const {
-        return lds_lane<P>(gstk[t] + (slot * W + c) * 32u * P);
+        return this->template S<W>(t, slot, c);
     }
     template <int W>
     __device__ __forceinline__ void put_g(int t, uint32_t slot, int c, const Vf<P> &v) const {
-        sts_lane<P>(gstk[t] + (slot * W + c) * 32u * P, v);
+        this->template put<W>(t, slot, c, v);
     }
     // adds the lane's counted points of g to the sum of flat parameter k
     // (points past the dataset's end may carry 0*inf = NaN adjoints)
@@ -80,7 +84,7 @@ struct RevIO : AccIO<P> {
 #pragma unroll
         for (int q = 0; q < P; ++q)
             if ((valid >> q) & 1u) s = s + g.v[q];
-        gacc[k * 32] += s;
+        sts_f32(gacc + 128u * k, lds_f32(gacc + 128u * k) + s);
     }
 };
 
@@ -471,23 +475,23 @@ __device__ __forceinline__ void fwd_op(Acc<PROF, P> &a, const RevIO<P> &io, uint
 static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec kinds at 29..32");
 #define RSR_SWITCH(M, EXTRA)                                                                          \
     if constexpr (PROF == P_F && (OMIT & 1)) {                                                        \
-        switch (kind) { EXTRA RSR_ADJ_F_NU(M) default: break; }                                       \
+        switch (kind) { EXTRA RSR_ADJ_F_NU(M) case K_STOP: return; default: __builtin_unreachable(); }                                       \
     } else if constexpr (PROF == P_F) {                                                               \
-        switch (kind) { EXTRA RSR_ADJ_F(M) default: break; }                                          \
+        switch (kind) { EXTRA RSR_ADJ_F(M) case K_STOP: return; default: __builtin_unreachable(); }                                          \
     } else if constexpr (PROF == P_FV3 && (OMIT & 3) == 3) {                                          \
-        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3_NM(M) default: break; }                      \
+        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3_NM(M) case K_STOP: return; default: __builtin_unreachable(); }                      \
     } else if constexpr (PROF == P_FV3 && (OMIT & 1)) {                                               \
-        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3(M) default: break; }                         \
+        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3(M) case K_STOP: return; default: __builtin_unreachable(); }                         \
     } else if constexpr (PROF == P_FV3 && (OMIT & 2)) {                                               \
-        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3_NM(M) default: break; }                         \
+        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3_NM(M) case K_STOP: return; default: __builtin_unreachable(); }                         \
     } else if constexpr (PROF == P_FV3) {                                                             \
-        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3(M) default: break; }                            \
+        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3(M) case K_STOP: return; default: __builtin_unreachable(); }                            \
     } else if constexpr (PROF == P_FV2M2 && (OMIT & 1)) {                                             \
-        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_X27(M, K_V2) RSR_X27(M, K_M2) default: break; }     \
+        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_X27(M, K_V2) RSR_X27(M, K_M2) case K_STOP: return; default: __builtin_unreachable(); }     \
     } else if constexpr (PROF == P_FV2M2) {                                                           \
-        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_X27(M, K_V2) RSR_X27(M, K_M2) default: break; }        \
+        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_X27(M, K_V2) RSR_X27(M, K_M2) case K_STOP: return; default: __builtin_unreachable(); }        \
     } else {                                                                                          \
-        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3(M) RSR_X27(M, K_M3) default: break; }           \
+        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3(M) RSR_X27(M, K_M3) case K_STOP: return; default: __builtin_unreachable(); }           \
     }
 #define RSR_TAPES                                                            \
     case kTapeKind[SF]: tape_store<PROF, P, SF>(a, io, arg); break;          \
@@ -498,30 +502,33 @@ static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec k
 #define RSR_NONE
 
 // Forward entries are (word, tape stores); the next entry is read while the
-// current one runs.
+// current one runs, and a K_STOP entry ends the sweep.  As in the register
+// kernel (kernels_reg.cu, run_program) the switch is a jump table over the
+// kinds the encoder can emit for the profile, without a range check.
 template <int PROF, int P, int OMIT>
-__device__ __forceinline__ void run_forward(Acc<PROF, P> &a, const RevIO<P> &io, const uint32_t *code, uint32_t n) {
-    uint32_t w = code[0], tapes = code[1];
-    for (uint32_t pc = 0; pc < n; ++pc) {
-        const uint32_t wn = code[2 * pc + 2], tn = code[2 * pc + 3];
-        const uint32_t arg = w >> 8, kind = w & 0xFFu;
+__device__ __forceinline__ void run_forward(Acc<PROF, P> &a, const RevIO<P> &io, uint32_t code) {
+    uint2 e = lds_u32x2(code);
+#pragma unroll 1
+    for (;;) {
+        code += 8u;
+        const uint2 en = lds_u32x2(code);
+        const uint32_t arg = e.x >> 8, kind = e.x & 0xFFu, tapes = e.y;
         RSR_SWITCH(RSR_F, RSR_TAPES)
-        w = wn;
-        tapes = tn;
+        e = en;
     }
 }
 
-// The next entry is read while the current one runs (the code ends with two
-// pad words).
+// The reverse entries, ended by K_STOP.
 template <int PROF, int P, int OMIT>
-__device__ __forceinline__ void run_reverse(Acc<PROF, P> &g, const RevIO<P> &io, const uint32_t *rev, uint32_t n) {
-    uint32_t w0 = rev[0], w1 = rev[1];
-    for (uint32_t i = 0; i < n; ++i) {
-        const uint32_t w0n = rev[2 * i + 2], w1n = rev[2 * i + 3];
-        const uint32_t arg = w0 >> 8, kind = w0 & 0xFFu;
+__device__ __forceinline__ void run_reverse(Acc<PROF, P> &g, const RevIO<P> &io, uint32_t code) {
+    uint2 e = lds_u32x2(code);
+#pragma unroll 1
+    for (;;) {
+        code += 8u;
+        const uint2 en = lds_u32x2(code);
+        const uint32_t arg = e.x >> 8, kind = e.x & 0xFFu, w1 = e.y;
         RSR_SWITCH(RSR_R, RSR_NONE)
-        w0 = w0n;
-        w1 = w1n;
+        e = en;
     }
 }
 
@@ -564,8 +571,9 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nw = blockDim.x >> 5;
     uint32_t *scode = reinterpret_cast<uint32_t *>(smem);
-    float *sconst = smem + ((a.smem_code_words + 2u + 3u) & ~3u);  // code and its two pad words
-    uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + ((a.smem_const_floats + 3u) & ~3u));  // [0] item, [1] tape
+    float *sconst = smem + ((a.smem_code_words + kAdjStopWords + 3u) & ~3u);  // code and its stop entries
+    // [0] item, [1] tape, [2..3] targets' byte distance from the features
+    uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + ((a.smem_const_floats + 3u) & ~3u));
     double *red = reinterpret_cast<double *>(meta + 4);  // [part][warp][1 + kAdjParams]
     float *wbase = smem + a.block_hdr_floats + (size_t)warp * a.region_floats;
 
@@ -576,8 +584,8 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
     __syncthreads();
     tm_fence_after_sync();
     RevIO<P> io;
-    io.consts = sconst;
-    io.tm = meta[1] + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(warp >> 2) * a.tmem_cols;
+    io.consts = opaque(smem_addr(sconst));
+    io.tm = opaque(meta[1] + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(warp >> 2) * a.tmem_cols);
 
     for (;;) {
         if (threadIdx.x == 0) meta[0] = atomicAdd(a.item_counter, 1u);
@@ -590,37 +598,35 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
             continue;
         }
         const ProgDesc pd = a.progs[it.prog_begin];
-        // this program's warp region: stacks | sums (n_tape: stack depths,
-        // 5 bits per type); the launch's region_floats is the largest of its
-        // programs'
+        // this program's warp region: stacks | gradient sums | Kahan state
+        // (n_tape: stack depths, 5 bits per type); the launch's region_floats
+        // is the largest of its programs'
         {
-            const uint32_t l0 = lane_point<P>(lane, 0);
-            uint32_t off = 0;
-            // A spilled value's adjoint takes the value's own slot: the one
-            // micro-op that pops the value reads it into registers (in both
-            // sweeps) before its reverse writes the adjoint, and no later
-            // reverse step reads the forward value (every PUSH has its own slot).
+            uint32_t at = smem_addr(wbase + lane_point<P>(lane, 0));
 #pragma unroll
             for (int t = 0; t < N_STACKS; ++t) {
-                io.stk[t] = wbase + off + l0;
-                io.gstk[t] = io.stk[t];
-                off += ((pd.n_tape >> (5 * t)) & 31u) * type_width(t) * 32u * P;
+                io.stk[t] = opaque(at);
+                at += ((pd.n_tape >> (5 * t)) & 31u) * type_width(t) * 128u * P;
             }
-            io.gacc = wbase + off + lane;
+            io.gacc = opaque(at + 4u * lane - 4u * lane_point<P>(lane, 0));
         }
         const uint32_t np = min(pd.n_consts, kAdjParams);
-        float *kahan = io.gacc - lane + np * 32u;  // [2][32], after the program's own gradient sums
-        for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) scode[i] = __ldg(a.code + pd.uop_off + i);
-        if (threadIdx.x == 0) scode[pd.uop_len] = scode[pd.uop_len + 1] = 0u;  // prefetch pads of the loops
-        for (uint32_t i = threadIdx.x; i < pd.n_consts; i += blockDim.x) sconst[i] = __ldg(a.consts + pd.const_off + i);
-        for (uint32_t k = 0; k < np; ++k) io.gacc[k * 32] = 0.0f;
-        kahan[lane] = 0.0f;
-        kahan[32 + lane] = 0.0f;
-        __syncthreads();
+        const uint32_t kahan = io.gacc + np * 128u;  // two rows: the running sum and its compensation
+        const uint32_t *gcode = a.code + pd.uop_off;
+        // the code, with a stop entry behind each sweep
+        const uint32_t cut = kAdjHeaderWords + 2u * __ldg(gcode);
+        for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) scode[i < cut ? i : i + 2u] = __ldg(gcode + i);
         const DatasetDesc ds = a.datasets[pd.dataset];
-        io.stride = (uint32_t)ds.stride;
-        const uint32_t n_fwd = scode[0], n_rev = scode[1];
-        const uint32_t *fwd = scode + kAdjHeaderWords, *rev = fwd + 2 * n_fwd;
+        if (threadIdx.x == 0) {
+            scode[cut] = scode[pd.uop_len + 2u] = K_STOP;
+            *reinterpret_cast<int64_t *>(meta + 2) =
+                reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
+        }
+        for (uint32_t i = threadIdx.x; i < pd.n_consts; i += blockDim.x) sconst[i] = __ldg(a.consts + pd.const_off + i);
+        for (uint32_t k = 0; k < np + 2u; ++k) sts_f32(io.gacc + 128u * k, 0.0f);
+        __syncthreads();
+        io.stride = opaque((uint32_t)ds.stride);
+        const uint32_t fwd = opaque(smem_addr(scode + kAdjHeaderWords)), rev = opaque(smem_addr(scode + cut + 2u));
         // The item's parts (kPartPoints points each) one after another; a
         // warp takes the same tiles of a part, and sums them the same way,
         // whatever the item's size, so a program's partial sums do not
@@ -632,15 +638,17 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
             for (uint32_t tile = it.tile_begin + part * part_tiles + warp; tile < part_end; tile += nw) {
                 const uint64_t t0 = (uint64_t)tile * (32u * P);
                 const uint64_t p0 = t0 + lane_point<P>(lane, 0);
-                io.xl = ds.x + p0;
+                io.xl = opaque(ds.x + p0);
                 uint32_t valid = 0;
 #pragma unroll
                 for (int q = 0; q < P; ++q) valid |= (t0 + lane_point<P>(lane, q) < ds.n_eval ? 1u : 0u) << q;
                 io.valid = valid;
                 Acc<PROF, P> acc;
-                run_forward<PROF, P, OMIT>(acc, io, fwd, n_fwd);
+                run_forward<PROF, P, OMIT>(acc, io, fwd);
                 tm_wait_st();  // the tape stores land before the reverse sweep reads them
-                const Vf<P> y = load_lane<P>(ds.y + p0);
+                const int64_t y_off = *reinterpret_cast<const volatile int64_t *>(meta + 2);
+                const Vf<P> y = load_lane<P>(
+                    reinterpret_cast<const float *>(reinterpret_cast<const char *>(io.xl) + y_off));
                 Acc<PROF, P> g;
                 g.F[0] = splat<P>(0.0f);
                 if constexpr (Types<PROF>::V2) zero_acc<P, 2>(g.V2);
@@ -648,8 +656,8 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                 if constexpr (Types<PROF>::M2) zero_acc<P, 4>(g.M2);
                 if constexpr (Types<PROF>::M3) zero_acc<P, 9>(g.M3);
                 Kahan ks;
-                ks.s = kahan[lane];
-                ks.c = kahan[32 + lane];
+                ks.s = lds_f32(kahan);
+                ks.c = lds_f32(kahan + 128u);
 #pragma unroll
                 for (int q = 0; q < P; ++q) {
                     const bool ok = (valid >> q) & 1u;
@@ -657,9 +665,9 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                     if (ok) ks.add(d * d);
                     g.F[0].v[q] = ok ? 2.0f * d : 0.0f;  // d(diff^2)/d pred, as in evaluator.rs:207
                 }
-                kahan[lane] = ks.s;
-                kahan[32 + lane] = ks.c;
-                run_reverse<PROF, P, OMIT>(g, io, rev, n_rev);
+                sts_f32(kahan, ks.s);
+                sts_f32(kahan + 128u, ks.c);
+                run_reverse<PROF, P, OMIT>(g, io, rev);
             }
             // the warp's sums of this part in f64, then a fresh start for the next
             {
@@ -667,14 +675,14 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                 // at a time, each as warp_sum adds
                 double *wred = red + ((size_t)part * nw + warp) * (1 + kAdjParams);
                 Kahan ks;
-                ks.s = kahan[lane];
-                ks.c = kahan[32 + lane];
+                ks.s = lds_f32(kahan);
+                ks.c = lds_f32(kahan + 128u);
                 for (uint32_t i0 = 0; i0 <= np; i0 += 4) {
                     double v[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const uint32_t i = i0 + j;
-                        v[j] = i == 0 ? (double)ks.value() : i <= np ? (double)io.gacc[(i - 1) * 32] : 0.0;
+                        v[j] = i == 0 ? (double)ks.value() : i <= np ? (double)lds_f32(io.gacc + 128u * (i - 1)) : 0.0;
                     }
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1)
@@ -685,9 +693,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                         for (int j = 0; j < 4; ++j)
                             if (i0 + j <= np) wred[i0 + j] = v[j];
                 }
-                for (uint32_t k = 0; k < np; ++k) io.gacc[k * 32] = 0.0f;
-                kahan[lane] = 0.0f;
-                kahan[32 + lane] = 0.0f;
+                for (uint32_t k = 0; k < np + 2u; ++k) sts_f32(io.gacc + 128u * k, 0.0f);
             }
         }
         // each part's sums across warps in a fixed order (the sums of the
@@ -709,7 +715,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
 }
 
 // ------------------------------------------------------------- launchers
-// Shared-memory layout (floats).  Block header: code (+2 pads) | constants |
+// Shared-memory layout (floats).  Block header: code (+ stop entries) | constants |
 // meta (4 words) | cross-warp sums (parts x warps x 33 doubles).  Per warp: stacks
 // (per type; the reverse sweep's adjoint stacks in the same slots) |
 // gradient sums (one row of 32 per parameter, at most 32) | Kahan state (2 x
@@ -731,7 +737,7 @@ uint32_t adj_pack_depth(const uint32_t *stack_depth) {
 
 void adj_layout(uint32_t code_words, uint32_t const_floats, uint32_t warp_floats, int nw, uint32_t parts,
                 LaunchArgs *a) {
-    a->block_hdr_floats = ((code_words + 2u + 3u) & ~3u) + ((const_floats + 3u) & ~3u) + 4u +
+    a->block_hdr_floats = ((code_words + kAdjStopWords + 3u) & ~3u) + ((const_floats + 3u) & ~3u) + 4u +
                           2u * parts * (uint32_t)nw * (1u + kAdjParams);
     a->region_floats = warp_floats;
     a->tmem_cols = 512u / ((uint32_t)nw / 4u);

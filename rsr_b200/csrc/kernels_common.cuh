@@ -143,32 +143,66 @@ __device__ __forceinline__ Vf<P> load_lane(const float *__restrict__ p) {
     }
 }
 
-// Shared-memory image of a lane's P values in a block of 32*P floats; p
-// points at the lane's first value (block start + lane_point(lane, 0)).
-template <int P>
-__device__ __forceinline__ Vf<P> lds_lane(const float *p) {
-    if constexpr (P <= 4) {
-        return *reinterpret_cast<const Vf<P> *>(p);
-    } else {
-        Vf<P> r;
-#pragma unroll
-        for (int j = 0; j < P / 4; ++j) {
-            const float4 a = *reinterpret_cast<const float4 *>(p + j * 128);
-            r.v[4 * j] = a.x; r.v[4 * j + 1] = a.y; r.v[4 * j + 2] = a.z; r.v[4 * j + 3] = a.w;
-        }
-        return r;
-    }
+// Shared memory by 32-bit address, for what an interpreter loop keeps in
+// registers across its switch.  ptxas may rebuild a value from what it came
+// from instead of holding it, and did so in the loop itself: a lane's feature
+// address from the thread index and a program's constants from the launch
+// arguments cost 10 of the 31 instructions of a one-constant micro-op at 80
+// registers (21 with both made opaque; vector workload 3.16 -> 2.91 ms).
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+__device__ __forceinline__ uint32_t opaque(uint32_t v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T *opaque(T *p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+    uint32_t r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ uint2 lds_u32x2(uint32_t a) {
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ void sts_f32(uint32_t a, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ float lds_f32(uint32_t a) { return __uint_as_float(lds_u32(a)); }
 
+// Shared-memory image of a lane's P values in a block of 32*P floats; a is
+// the address of the lane's first value (block start + lane_point(lane, 0)).
 template <int P>
-__device__ __forceinline__ void sts_lane(float *p, const Vf<P> &v) {
-    if constexpr (P <= 4) {
-        *reinterpret_cast<Vf<P> *>(p) = v;
+__device__ __forceinline__ Vf<P> lds_lane(uint32_t a) {
+    Vf<P> r;
+    if constexpr (P == 2) {
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "r"(a));
     } else {
 #pragma unroll
         for (int j = 0; j < P / 4; ++j)
-            *reinterpret_cast<float4 *>(p + j * 128) = make_float4(v.v[4 * j], v.v[4 * j + 1], v.v[4 * j + 2],
-                                                                  v.v[4 * j + 3]);
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(r.v[4 * j]), "=f"(r.v[4 * j + 1]), "=f"(r.v[4 * j + 2]), "=f"(r.v[4 * j + 3])
+                         : "r"(a + 512u * j));
+    }
+    return r;
+}
+
+template <int P>
+__device__ __forceinline__ void sts_lane(uint32_t a, const Vf<P> &v) {
+    if constexpr (P == 2) {
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.v[0]), "f"(v.v[1]) : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < P / 4; ++j)
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a + 512u * j), "f"(v.v[4 * j]),
+                         "f"(v.v[4 * j + 1]), "f"(v.v[4 * j + 2]), "f"(v.v[4 * j + 3])
+                         : "memory");
     }
 }
 

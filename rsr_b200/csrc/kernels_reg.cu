@@ -39,47 +39,47 @@ static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec k
 #define RSR_BLOCK_M2 RSR_C27(K_M2)   // 104..130
 #define RSR_BLOCK_M3 RSR_C27(K_M3)   // 136..162
 
-// Runs one program (accumulator form) on this lane's P points; the result
-// is left in A_F.  OMIT: handlers left out of the kernel because no program
-// of the launch needs them -- bit 0: the unary Float ops (sin, cos, exp,
-// sqr, sqrt, ln); bit 1 (F+V3 profile): mat-vec products whose matrix is a
-// feature, a constant or a spilled value.
+// Runs one program (accumulator form, ended by a K_STOP word) on this lane's
+// P points; the result is left in A_F.  OMIT: handlers left out of the kernel
+// because no program of the launch needs them -- bit 0: the unary Float ops
+// (sin, cos, exp, sqr, sqrt, ln); bit 1 (F+V3 profile): mat-vec products whose
+// matrix is a feature, a constant or a spilled value.
+//
+// What bounds it is the dispatch around the P x width FP32 instructions of a
+// micro-op, so the loop holds nothing else: the switch is a jump table
+// (built with --jump-table-density, build.py) over the kinds the encoder can
+// emit for the profile, with no range check (the default is unreachable), and
+// the program ends by a micro-op instead of a counter.
+#define RSR_RUN(CASES)                                                   \
+    switch (w & 0xFFu) {                                                 \
+        CASES                                                            \
+        case K_STOP: return;                                             \
+        default: __builtin_unreachable();                                \
+    }
 template <int PROF, int P, int OMIT>
-__device__ __forceinline__ void run_program(Acc<PROF, P> &a, const AccIO<P> &io, const uint32_t *code,
-                                            uint32_t len) {
-    // Each profile's switch lists only its own types' kinds, so the branch
-    // tree the compiler builds for it is as shallow as the profile allows.
-    uint32_t w = code[0];
-    for (uint32_t pc = 0; pc < len; ++pc) {
-        const uint32_t wn = code[pc + 1];
+__device__ __forceinline__ void run_program(Acc<PROF, P> &a, const AccIO<P> &io, uint32_t code) {
+    constexpr bool NU = (OMIT & 1) != 0, NM = (OMIT & 2) != 0;
+    uint32_t w = lds_u32(code);
+#pragma unroll 1
+    for (;;) {
+        code += 4u;
+        const uint32_t wn = lds_u32(code);  // the word after K_STOP is read, not run
         const uint32_t arg = w >> 8;
-        const uint32_t kind = w & 0xFFu;
-        constexpr bool NU = (OMIT & 1) != 0, NM = (OMIT & 2) != 0;
-        if constexpr (PROF == P_F && NU) {
-            switch (kind) { RSR_BLOCK_F_NU default: break; }
-        } else if constexpr (PROF == P_F) {
-            switch (kind) { RSR_BLOCK_F default: break; }
-        } else if constexpr (PROF == P_FV3 && NU && NM) {
-            switch (kind) { RSR_BLOCK_F_NU RSR_BLOCK_V3_NM default: break; }
-        } else if constexpr (PROF == P_FV3 && NU) {
-            switch (kind) { RSR_BLOCK_F_NU RSR_BLOCK_V3_F default: break; }
-        } else if constexpr (PROF == P_FV3 && NM) {
-            switch (kind) { RSR_BLOCK_F RSR_BLOCK_V3_NM default: break; }
-        } else if constexpr (PROF == P_FV3) {
-            switch (kind) { RSR_BLOCK_F RSR_BLOCK_V3_F default: break; }
-        } else if constexpr (PROF == P_FV2M2 && NU) {
-            switch (kind) { RSR_BLOCK_F_NU RSR_BLOCK_V2 RSR_BLOCK_M2 default: break; }
-        } else if constexpr (PROF == P_FV2M2) {
-            switch (kind) { RSR_BLOCK_F RSR_BLOCK_V2 RSR_BLOCK_M2 default: break; }
-        } else if constexpr (PROF == P_FV3M3) {
-            switch (kind) { RSR_BLOCK_F RSR_BLOCK_V3 RSR_BLOCK_M3 default: break; }
-        } else {
-            switch (kind) { RSR_BLOCK_F RSR_BLOCK_V2 RSR_BLOCK_V3 RSR_BLOCK_M2 RSR_BLOCK_M3 default: break; }
-        }
+        if constexpr (PROF == P_F && NU) { RSR_RUN(RSR_BLOCK_F_NU) }
+        else if constexpr (PROF == P_F) { RSR_RUN(RSR_BLOCK_F) }
+        else if constexpr (PROF == P_FV3 && NU && NM) { RSR_RUN(RSR_BLOCK_F_NU RSR_BLOCK_V3_NM) }
+        else if constexpr (PROF == P_FV3 && NU) { RSR_RUN(RSR_BLOCK_F_NU RSR_BLOCK_V3_F) }
+        else if constexpr (PROF == P_FV3 && NM) { RSR_RUN(RSR_BLOCK_F RSR_BLOCK_V3_NM) }
+        else if constexpr (PROF == P_FV3) { RSR_RUN(RSR_BLOCK_F RSR_BLOCK_V3_F) }
+        else if constexpr (PROF == P_FV2M2 && NU) { RSR_RUN(RSR_BLOCK_F_NU RSR_BLOCK_V2 RSR_BLOCK_M2) }
+        else if constexpr (PROF == P_FV2M2) { RSR_RUN(RSR_BLOCK_F RSR_BLOCK_V2 RSR_BLOCK_M2) }
+        else if constexpr (PROF == P_FV3M3) { RSR_RUN(RSR_BLOCK_F RSR_BLOCK_V3 RSR_BLOCK_M3) }
+        else { RSR_RUN(RSR_BLOCK_F RSR_BLOCK_V2 RSR_BLOCK_V3 RSR_BLOCK_M2 RSR_BLOCK_M3) }
         w = wn;
     }
 }
 
+#undef RSR_RUN
 #undef RSR_BLOCK_F
 #undef RSR_BLOCK_F_NU
 #undef RSR_BLOCK_V3_NM
@@ -130,14 +130,17 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
     const int nw = blockDim.x >> 5;
     uint32_t *scode = reinterpret_cast<uint32_t *>(smem);
     float *sconst = smem + align4r(a.smem_code_words);
-    uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + align4r(a.smem_const_floats));  // [g][3], [24] item
+    // [g][2] code and constants of each program, [24] item, [25] its
+    // programs, [26..27] targets' byte distance from the features, [28..29]
+    // points to count, [30] last tile, [31] first program
+    uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + align4r(a.smem_const_floats));
     double *red = reinterpret_cast<double *>(meta + 32);                                  // [warp][g]
     float *wbase = smem + a.block_hdr_floats + (size_t)warp * a.region_floats;
     float *sacc = wbase + a.acc_off;  // [g][2][32] Kahan state of this warp
 
     AccIO<P> io;
 #pragma unroll
-    for (int t = 0; t < N_STACKS; ++t) io.stk[t] = wbase + a.stack_off[t] + lane_point<P>(lane, 0);
+    for (int t = 0; t < N_STACKS; ++t) io.stk[t] = opaque(smem_addr(wbase + a.stack_off[t] + lane_point<P>(lane, 0)));
 
     for (;;) {
         if (threadIdx.x == 0) meta[24] = atomicAdd(a.item_counter, 1u);
@@ -156,50 +159,61 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
                 continue;
             }
         }
+        const DatasetDesc ds = a.datasets[a.progs[it.prog_begin].dataset];
         if (threadIdx.x == 0) {
             uint32_t coff = 0, koff = 0;
             for (uint32_t g = 0; g < G; ++g) {
                 const ProgDesc pd = a.progs[it.prog_begin + g];
-                meta[3 * g] = coff;
-                meta[3 * g + 1] = pd.uop_len;
-                meta[3 * g + 2] = koff;
-                scode[coff + pd.uop_len] = 0u;  // prefetch pad
+                meta[2 * g] = coff;
+                meta[2 * g + 1] = koff;
+                scode[coff + pd.uop_len] = K_STOP;
                 coff += pd.uop_len + 1;
                 koff += pd.n_consts;
             }
+            *reinterpret_cast<int64_t *>(meta + 26) =
+                reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
+            *reinterpret_cast<uint64_t *>(meta + 28) = ds.n_eval;
+            meta[25] = G;
+            meta[30] = it.tile_end;
+            meta[31] = it.prog_begin;
         }
         __syncthreads();
         for (uint32_t g = 0; g < G; ++g) {
             const ProgDesc pd = a.progs[it.prog_begin + g];
-            for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) scode[meta[3 * g] + i] = __ldg(a.code + pd.uop_off + i);
+            for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) scode[meta[2 * g] + i] = __ldg(a.code + pd.uop_off + i);
             for (uint32_t i = threadIdx.x; i < pd.n_consts; i += blockDim.x)
-                sconst[meta[3 * g + 2] + i] = __ldg(a.consts + pd.const_off + i);
+                sconst[meta[2 * g + 1] + i] = __ldg(a.consts + pd.const_off + i);
             sacc[(g * 2) * 32 + lane] = 0.0f;
             sacc[(g * 2 + 1) * 32 + lane] = 0.0f;
         }
         __syncthreads();
-        const DatasetDesc ds = a.datasets[a.progs[it.prog_begin].dataset];
-        io.stride = (uint32_t)ds.stride;
+        io.stride = opaque((uint32_t)ds.stride);
         Acc<PROF, P> acc;
-        for (uint32_t tile = it.tile_begin + warp; tile < it.tile_end; tile += nw) {
-            const uint64_t t0 = (uint64_t)tile * (32u * P);
-            const uint64_t p0 = t0 + lane_point<P>(lane, 0);
-            io.xl = ds.x + p0;
-            const Vf<P> y = load_lane<P>(ds.y + p0);
-            const bool full = t0 + lane_point<P>(lane, P - 1) < ds.n_eval;  // the lane's last value
-            for (uint32_t g = 0; g < G; ++g) {
-                if (a.active && !a.active[it.prog_begin + g]) continue;
-                io.consts = sconst + meta[3 * g + 2];
-                run_program<PROF, P, OMIT>(acc, io, scode + meta[3 * g], meta[3 * g + 1]);
+        // What the loops need beside the program itself -- their bounds, the
+        // targets, the dataset's end -- is read again for every program
+        // (shared memory and L1): held in registers it would be live across
+        // the interpreter, which has none to spare at three blocks an SM.
+        const volatile uint32_t *vmeta = meta;
+        for (uint32_t tile = it.tile_begin + warp; tile < vmeta[30]; tile += nw) {
+            io.xl = opaque(ds.x + ((uint64_t)tile * (32u * P) + lane_point<P>(lane, 0)));
+            for (uint32_t g = 0; g < vmeta[25]; ++g) {
+                if (a.active && !a.active[vmeta[31] + g]) continue;
+                io.consts = opaque(smem_addr(sconst + meta[2 * g + 1]));
+                run_program<PROF, P, OMIT>(acc, io, opaque(smem_addr(scode + meta[2 * g])));
                 const Vf<P> pred = acc.F[0];
+                const int64_t y_off = *reinterpret_cast<const volatile int64_t *>(vmeta + 26);
+                const uint64_t n_eval = *reinterpret_cast<const volatile uint64_t *>(vmeta + 28);
+                const uint64_t t0 = (uint64_t)tile * (32u * P);
                 if (a.mode == MODE_POINTS) {
-                    store_lane<P>(a.points_out + (uint64_t)(it.prog_begin + g) * a.points_stride + t0, lane, pred,
-                                  t0, ds.n_eval);
+                    store_lane<P>(a.points_out + (uint64_t)(vmeta[31] + g) * a.points_stride + t0, lane, pred,
+                                  t0, n_eval);
                 } else {
+                    const Vf<P> y = load_lane<P>(
+                        reinterpret_cast<const float *>(reinterpret_cast<const char *>(io.xl) + y_off));
                     Kahan k;
                     k.s = sacc[(g * 2) * 32 + lane];
                     k.c = sacc[(g * 2 + 1) * 32 + lane];
-                    if (full) {
+                    if (t0 + lane_point<P>(lane, P - 1) < n_eval) {
                         // the lane's P squared errors summed pairwise, then one
                         // compensated add per tile
                         float sq[P];
@@ -216,7 +230,7 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
                     } else {
 #pragma unroll
                         for (int q = 0; q < P; ++q) {
-                            if (t0 + lane_point<P>(lane, q) < ds.n_eval) {
+                            if (t0 + lane_point<P>(lane, q) < n_eval) {
                                 const float d = pred.v[q] - y.v[q];
                                 k.add(d * d);
                             }
