@@ -54,12 +54,24 @@ struct RevIO : AccIO<P> {
     uint32_t tm;            // tensor-memory tape: this warp's lanes, column 0
     uint32_t gacc;          // shared-memory address of this lane's f32 gradient sums, one row of 32 a parameter
     uint32_t valid;         // bit q: value q of the lane is a counted point
-    // a tape reference (uops.h, kTapeRefX): a tape slot, or the feature or
-    // constant the forward value was loaded from
+    // a tape reference (uops.h, kTapeRefX) of a value of W components: tape
+    // slots, or the features or constants the forward value was loaded from
+    template <int W>
+    __device__ __forceinline__ void T(Vf<P> *v, uint32_t ref) const {
+        if (ref & kTapeRefX) {
+#pragma unroll
+            for (int c = 0; c < W; ++c) v[c] = this->X((ref & kTapeRefIndex) + c);
+        } else if (ref & kTapeRefC) {
+#pragma unroll
+            for (int c = 0; c < W; ++c) v[c] = this->C((ref & kTapeRefIndex) + c);
+        } else {
+            tm_ld<P, W>(v, tm + ref * (uint32_t)P);
+        }
+    }
     __device__ __forceinline__ Vf<P> T(uint32_t ref) const {
-        if (ref & kTapeRefX) return this->X(ref & kTapeRefIndex);
-        if (ref & kTapeRefC) return this->C(ref & kTapeRefIndex);
-        return tm_ld<P>(tm + ref * (uint32_t)P);
+        Vf<P> v;
+        T<1>(&v, ref);
+        return v;
     }
     __device__ __forceinline__ void put_tape(uint32_t slot, const Vf<P> &v) const {
         tm_st<P>(tm + slot * (uint32_t)P, v);
@@ -76,15 +88,50 @@ struct RevIO : AccIO<P> {
     __device__ __forceinline__ void put_g(int t, uint32_t slot, int c, const Vf<P> &v) const {
         this->template put<W>(t, slot, c, v);
     }
-    // adds the lane's counted points of g to the sum of flat parameter k
-    // (points past the dataset's end may carry 0*inf = NaN adjoints)
+    // Adds the lane's counted points of g, in order, to the sum of flat
+    // parameter k (points past the dataset's end may carry 0*inf = NaN
+    // adjoints); parameters from kAdjParams on share a row nobody reads.
+    // One asm statement, so that nvcc sees no branch here: with one it kept
+    // copies of the adjoints for the merge behind it, and the reverse loop
+    // moved accumulators in every entry (32 of 36 instructions of one that
+    // does nothing).
     __device__ __forceinline__ void grad_add(uint32_t k, const Vf<P> &g) const {
-        if (k >= kAdjParams) return;
-        float s = 0.0f;
-#pragma unroll
-        for (int q = 0; q < P; ++q)
-            if ((valid >> q) & 1u) s = s + g.v[q];
-        sts_f32(gacc + 128u * k, lds_f32(gacc + 128u * k) + s);
+        const uint32_t row = gacc + 128u * min(k, kAdjParams);
+        if constexpr (P == 2) {
+            asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\n"
+                         "and.b32 b, %3, 1;\nsetp.ne.u32 p, b, 0;\nmov.f32 s, 0f00000000;\n@p add.rn.f32 s, s, %1;\n"
+                         "and.b32 b, %3, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
+                         "ld.shared.f32 o, [%0];\nadd.rn.f32 o, o, s;\nst.shared.f32 [%0], o;\n}"
+                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "r"(valid) : "memory");
+        } else if constexpr (P == 4) {
+            asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
+                         "mov.f32 s, 0f00000000;\nsetp.ne.u32 p, %5, 15;\n@p bra PART;\n"
+                         "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\nbra DONE;\n"
+                         "PART:\n"
+                         "and.b32 b, %5, 1;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %1;\n"
+                         "and.b32 b, %5, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
+                         "and.b32 b, %5, 4;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %3;\n"
+                         "and.b32 b, %5, 8;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %4;\n"
+                         "DONE:\nadd.rn.f32 o, o, s;\nst.shared.f32 [%0], o;\n}"
+                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "r"(valid) : "memory");
+        } else {
+            asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
+                         "mov.f32 s, 0f00000000;\nsetp.ne.u32 p, %9, 255;\n@p bra PART;\n"
+                         "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\n"
+                         "add.rn.f32 s, s, %5;\nadd.rn.f32 s, s, %6;\nadd.rn.f32 s, s, %7;\nadd.rn.f32 s, s, %8;\nbra DONE;\n"
+                         "PART:\n"
+                         "and.b32 b, %9, 1;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %1;\n"
+                         "and.b32 b, %9, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
+                         "and.b32 b, %9, 4;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %3;\n"
+                         "and.b32 b, %9, 8;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %4;\n"
+                         "and.b32 b, %9, 16;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %5;\n"
+                         "and.b32 b, %9, 32;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %6;\n"
+                         "and.b32 b, %9, 64;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %7;\n"
+                         "and.b32 b, %9, 128;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %8;\n"
+                         "DONE:\nadd.rn.f32 o, o, s;\nst.shared.f32 [%0], o;\n}"
+                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "f"(g.v[4]), "f"(g.v[5]),
+                         "f"(g.v[6]), "f"(g.v[7]), "r"(valid) : "memory");
+        }
     }
 };
 
@@ -101,8 +148,7 @@ __device__ __forceinline__ void zero_acc(Vf<P> *G) {
 
 template <int P, int W>
 __device__ __forceinline__ void load_tape(Vf<P> *v, const RevIO<P> &io, uint32_t slot) {
-#pragma unroll
-    for (int c = 0; c < W; ++c) v[c] = io.T(slot + c);
+    io.template T<W>(v, slot);
 }
 
 // The adjoint of a second operand from source SRC: a constant's goes to the
@@ -453,11 +499,11 @@ __device__ __forceinline__ void fwd_op(Acc<PROF, P> &a, const RevIO<P> &io, uint
     constexpr int t = K >= K_M3 ? SM3 : K >= K_M2 ? SM2 : K >= K_V3 ? SV3 : K >= K_V2 ? SV2 : SF;
     if ((tapes & kNoTape) != kNoTape) tape_store<PROF, P, t>(a, io, tapes & kNoTape);
     acc_op<PROF, P, K>(a, io, arg);
-    if ((tapes >> 16) != kNoTape) tape_store<PROF, P, t>(a, io, tapes >> 16);
+    if (tapes < (kNoTape << 16)) tape_store<PROF, P, t>(a, io, tapes >> 16);
 }
 
-#define RSR_F(K) case (K): fwd_op<PROF, P, (K)>(a, io, arg, tapes); break;
-#define RSR_R(K) case (K): rev_op<PROF, P, (K)>(g, io, arg, w1); break;
+#define RSR_F(K) case (K): fwd_op<PROF, P, (K)>(a, io, arg, tapes); handler_end<(K)>(); break;
+#define RSR_R(K) case (K): rev_op<PROF, P, (K)>(g, io, arg, w1); handler_end<(K)>(); break;
 #define RSR_X4(M, K) M(K) M(K + 1) M(K + 2) M(K + 3)
 #define RSR_X9(M, K) RSR_X4(M, K) RSR_X4(M, K + 4) M(K + 8)
 #define RSR_X27(M, K) RSR_X9(M, K) RSR_X9(M, K + 9) RSR_X9(M, K + 18)
@@ -549,8 +595,8 @@ __device__ __forceinline__ void run_reverse(Acc<PROF, P> &g, const RevIO<P> &io,
 // Block-cooperative persistent kernel, one block per SM: its warps take the
 // tiles of one work item (one program on a chunk of points).  Shared
 // memory: block header (code | constants | meta | cross-warp sums), then
-// one region per warp: stacks (then adjoint stacks) | gradient sums | Kahan
-// state.  The tape is in tensor memory, a.tmem_cols columns per warp.
+// one region per warp: stacks (then adjoint stacks) | gradient sums | squared
+// errors.  The tape is in tensor memory, a.tmem_cols columns per warp.
 // Warps of a block of instance (PROF, P), one block per SM: a multiple of
 // 4, at most 16.  More warps than the instance's registers allow unspilled
 // pay: the extra warps hide more of the dispatch latency than the spill
@@ -598,7 +644,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
             continue;
         }
         const ProgDesc pd = a.progs[it.prog_begin];
-        // this program's warp region: stacks | gradient sums | Kahan state
+        // this program's warp region: stacks | gradient sums | squared errors
         // (n_tape: stack depths, 5 bits per type); the launch's region_floats
         // is the largest of its programs'
         {
@@ -611,7 +657,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
             io.gacc = opaque(at + 4u * lane - 4u * lane_point<P>(lane, 0));
         }
         const uint32_t np = min(pd.n_consts, kAdjParams);
-        const uint32_t kahan = io.gacc + np * 128u;  // two rows: the running sum and its compensation
+        const uint32_t sse = io.gacc + 4u * lane + (np + (pd.n_consts > kAdjParams)) * 128u;  // this lane's squared errors (f64, a row of 256 bytes)
         const uint32_t *gcode = a.code + pd.uop_off;
         // the code, with a stop entry behind each sweep
         const uint32_t cut = kAdjHeaderWords + 2u * __ldg(gcode);
@@ -623,7 +669,8 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                 reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
         }
         for (uint32_t i = threadIdx.x; i < pd.n_consts; i += blockDim.x) sconst[i] = __ldg(a.consts + pd.const_off + i);
-        for (uint32_t k = 0; k < np + 2u; ++k) sts_f32(io.gacc + 128u * k, 0.0f);
+        for (uint32_t k = 0; k < np; ++k) sts_f32(io.gacc + 128u * k, 0.0f);
+        sts_f64(sse, 0.0);
         __syncthreads();
         io.stride = opaque((uint32_t)ds.stride);
         const uint32_t fwd = opaque(smem_addr(scode + kAdjHeaderWords)), rev = opaque(smem_addr(scode + cut + 2u));
@@ -639,9 +686,12 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                 const uint64_t t0 = (uint64_t)tile * (32u * P);
                 const uint64_t p0 = t0 + lane_point<P>(lane, 0);
                 io.xl = opaque(ds.x + p0);
-                uint32_t valid = 0;
+                uint32_t valid = (1u << P) - 1u;
+                if (t0 + 32u * P > ds.n_eval) {
+                    valid = 0;
 #pragma unroll
-                for (int q = 0; q < P; ++q) valid |= (t0 + lane_point<P>(lane, q) < ds.n_eval ? 1u : 0u) << q;
+                    for (int q = 0; q < P; ++q) valid |= (t0 + lane_point<P>(lane, q) < ds.n_eval ? 1u : 0u) << q;
+                }
                 io.valid = valid;
                 Acc<PROF, P> acc;
                 run_forward<PROF, P, OMIT>(acc, io, fwd);
@@ -655,45 +705,45 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                 if constexpr (Types<PROF>::V3) zero_acc<P, 3>(g.V3);
                 if constexpr (Types<PROF>::M2) zero_acc<P, 4>(g.M2);
                 if constexpr (Types<PROF>::M3) zero_acc<P, 9>(g.M3);
-                Kahan ks;
-                ks.s = lds_f32(kahan);
-                ks.c = lds_f32(kahan + 128u);
+                double sq = lds_f64(sse);
 #pragma unroll
                 for (int q = 0; q < P; ++q) {
                     const bool ok = (valid >> q) & 1u;
                     const float d = acc.F[0].v[q] - y.v[q];
-                    if (ok) ks.add(d * d);
+                    if (ok) sq += (double)(d * d);
                     g.F[0].v[q] = ok ? 2.0f * d : 0.0f;  // d(diff^2)/d pred, as in evaluator.rs:207
                 }
-                sts_f32(kahan, ks.s);
-                sts_f32(kahan + 128u, ks.c);
+                sts_f64(sse, sq);
                 run_reverse<PROF, P, OMIT>(g, io, rev);
             }
-            // the warp's sums of this part in f64, then a fresh start for the next
+            // The warp's sums of this part in f64, then a fresh start for the
+            // next.  The gradient rows are summed across lanes eight at a
+            // time: four lanes take a row, eight of its values each (value
+            // (8 j + i + row) mod 32 in step i, every lane in its own bank),
+            // then add theirs up.  A row by itself, every lane in five
+            // exchange steps, is 3.5 times the instructions (15 x 8 against
+            // 8 x 3 + 6), on a part of one tile a warp.
             {
-                // sums 0 (squared errors) .. np (gradient), four warp sums
-                // at a time, each as warp_sum adds
                 double *wred = red + ((size_t)part * nw + warp) * (1 + kAdjParams);
-                Kahan ks;
-                ks.s = lds_f32(kahan);
-                ks.c = lds_f32(kahan + 128u);
-                for (uint32_t i0 = 0; i0 <= np; i0 += 4) {
-                    double v[4];
+                const double e = warp_sum(lds_f64(sse));
+                if (lane == 0) wred[0] = e;
+                __syncwarp();
+                const uint32_t row0 = (uint32_t)lane >> 2;
+                for (uint32_t base = 0; base < np; base += 8) {
+                    const uint32_t row = base + row0;
+                    double v = 0.0;
+                    if (row < np) {
+                        const uint32_t at = io.gacc - 4u * lane + 128u * row;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint32_t i = i0 + j;
-                        v[j] = i == 0 ? (double)ks.value() : i <= np ? (double)lds_f32(io.gacc + 128u * (i - 1)) : 0.0;
+                        for (uint32_t i = 0; i < 8; ++i) v += (double)lds_f32(at + ((4u * (8u * (lane & 3u) + i + row0)) & 127u));
                     }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-                    if (lane == 0)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (i0 + j <= np) wred[i0 + j] = v[j];
+                    v += __shfl_xor_sync(0xffffffffu, v, 1);
+                    v += __shfl_xor_sync(0xffffffffu, v, 2);
+                    if ((lane & 3) == 0 && row < np) wred[1 + row] = v;
                 }
-                for (uint32_t k = 0; k < np + 2u; ++k) sts_f32(io.gacc + 128u * k, 0.0f);
+                __syncwarp();
+                for (uint32_t k = 0; k < np; ++k) sts_f32(io.gacc + 128u * k, 0.0f);
+                sts_f64(sse, 0.0);
             }
         }
         // each part's sums across warps in a fixed order (the sums of the
@@ -718,14 +768,15 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
 // Shared-memory layout (floats).  Block header: code (+ stop entries) | constants |
 // meta (4 words) | cross-warp sums (parts x warps x 33 doubles).  Per warp: stacks
 // (per type; the reverse sweep's adjoint stacks in the same slots) |
-// gradient sums (one row of 32 per parameter, at most 32) | Kahan state (2 x
-// 32), each program's own sizes (the kernel lays the region out per item);
+// gradient sums (one row of 32 per parameter, at most 32, and one for all
+// parameters past them) | squared errors (a
+// row of 32 doubles), each program's own sizes (the kernel lays the region out per item);
 // warp_floats is the largest region of the launch.  The tape is in tensor
 // memory (a.tmem_cols columns a warp).
 uint32_t adj_warp_floats(const uint32_t *stack_depth, int P, uint32_t n_params) {
     uint32_t slots = 0;  // the stacks, whose slots the adjoints reuse
     for (int t = 0; t < N_STACKS; ++t) slots += stack_depth[t] * (uint32_t)kStackWidth[t];
-    const uint32_t np = n_params < kAdjParams ? n_params : kAdjParams;
+    const uint32_t np = n_params <= kAdjParams ? n_params : kAdjParams + 1;
     return (slots * 32u * (uint32_t)P + np * 32u + 2u * 32u + 3u) & ~3u;
 }
 

@@ -20,7 +20,7 @@
 
 namespace rsr {
 
-#define RSR_C(K) case (K): acc_op<PROF, P, (K)>(a, io, arg); break;
+#define RSR_C(K) case (K): acc_op<PROF, P, (K)>(a, io, arg); handler_end<(K)>(); break;
 #define RSR_C4(K) RSR_C(K) RSR_C(K + 1) RSR_C(K + 2) RSR_C(K + 3)
 #define RSR_C9(K) RSR_C4(K) RSR_C4(K + 4) RSR_C(K + 8)
 #define RSR_C27(K) RSR_C9(K) RSR_C9(K + 9) RSR_C9(K + 18)

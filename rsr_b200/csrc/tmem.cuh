@@ -45,29 +45,35 @@ __device__ __forceinline__ void tm_st(uint32_t addr, const Vf<P> &v) {
     }
 }
 
-// The wait names the loaded registers, so no use of them is scheduled
-// before it.
 template <int P>
-__device__ __forceinline__ Vf<P> tm_ld(uint32_t addr) {
-    uint32_t r[P];
+__device__ __forceinline__ void tm_ld_issue(Vf<P> &v, uint32_t addr) {
     if constexpr (P == 2) {
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr) : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1])::"memory");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=f"(v.v[0]), "=f"(v.v[1]) : "r"(addr) : "memory");
     } else if constexpr (P == 4) {
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])::"memory");
+                     : "=f"(v.v[0]), "=f"(v.v[1]), "=f"(v.v[2]), "=f"(v.v[3]) : "r"(addr) : "memory");
     } else {
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "=f"(v.v[0]), "=f"(v.v[1]), "=f"(v.v[2]), "=f"(v.v[3]), "=f"(v.v[4]), "=f"(v.v[5]), "=f"(v.v[6]), "=f"(v.v[7])
                      : "r"(addr) : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;"
-                     : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
     }
-    Vf<P> v;
+}
+// Names v's registers: no use of them is scheduled before the asm
+// statements above this one.
+template <int P>
+__device__ __forceinline__ void tm_pin(Vf<P> &v) {
 #pragma unroll
-    for (int j = 0; j < P; ++j) v.v[j] = __uint_as_float(r[j]);
-    return v;
+    for (int j = 0; j < P; ++j) asm volatile("" : "+f"(v.v[j]));
+}
+// W slots of P columns each from addr on: the loads in flight together, one
+// wait, and the registers named after it.
+template <int P, int W>
+__device__ __forceinline__ void tm_ld(Vf<P> *v, uint32_t addr) {
+#pragma unroll
+    for (int c = 0; c < W; ++c) tm_ld_issue<P>(v[c], addr + c * (uint32_t)P);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int c = 0; c < W; ++c) tm_pin<P>(v[c]);
 }
 
 }  // namespace rsr
