@@ -39,7 +39,11 @@ struct AccIO {
     uint32_t stride;        // floats between features
     uint32_t consts;        // shared-memory address of the program's constants
     uint32_t stk[N_STACKS]; // per-type stacks (shared-memory addresses), block (slot*W + c), at this lane's first value
-    __device__ __forceinline__ Vf<P> X(uint32_t f) const { return load_lane<P>(xl + (size_t)f * stride); }
+    // 4f * stride bytes in one wide multiply-add (f * stride floats is one, and
+    // a 64-bit shift and add)
+    __device__ __forceinline__ Vf<P> X(uint32_t f) const {
+        return load_lane<P>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(xl) + (uint64_t)(4u * f) * stride));
+    }
     __device__ __forceinline__ Vf<P> C(uint32_t i) const { return splat<P>(lds_f32(consts + 4u * i)); }
     template <int W>
     __device__ __forceinline__ Vf<P> S(int t, uint32_t slot, int c) const {
