@@ -122,6 +122,7 @@ struct Node {
     int pos = 0;         // reference stack position of the result
     bool stale = false;  // LoadConst of a mismatched variant: writes nothing
     int alias = -1;      // stale: node whose value sits in that slot (-1: zero)
+    bool is_const = false;  // every leaf under it is a constant
 };
 
 bool leaf(const Node &n) { return is_load(n.opcode) && !n.stale; }
@@ -175,6 +176,8 @@ struct Scratch {
     std::vector<int> idx, pos, vend, astart;
     std::vector<uint32_t> vs, as;
     SlotPool vals;
+    std::vector<int> hoist;             // FORM_HOIST
+    std::vector<Node> hoisted_nodes;
 };
 thread_local Scratch tls;
 
@@ -515,6 +518,7 @@ class AccEmitter {
 
     uint32_t writes_of(int id) const { return writes_[id]; }
     int size_of(int id) const { return size_[id]; }
+    void emit(int kind, uint32_t arg) { code.push_back(uop_word((uint32_t)kind, arg)); }
 
     std::vector<uint32_t> &code;
     int max_sp[N_STACKS] = {0, 0, 0, 0, 0};
@@ -553,13 +557,17 @@ class AccEmitter {
         return slot;
     }
     void pop(int t) { sp_[t]--; }
-    void emit(int kind, uint32_t arg) { code.push_back(uop_word((uint32_t)kind, arg)); }
 
     const std::vector<Node> &nodes_;
     std::vector<uint32_t> &writes_;
     std::vector<int> &size_;
     int sp_[N_STACKS] = {0, 0, 0, 0, 0};
 };
+
+int const_load_of(int t) {
+    return t == SF ? LOAD_CONST_F : t == SV2 ? LOAD_CONST_V2 : t == SV3 ? LOAD_CONST_V3 : t == SM2 ? LOAD_CONST_M2
+                                                                                                : LOAD_CONST_M3;
+}
 
 // Register-adjoint code (uops.h, kAdjHeaderWords) of a tree an AccEmitter
 // has analysed: the accumulator form's evaluation order, a load directly
@@ -946,6 +954,7 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
                     n.alias = p < kRefStackSlots ? last[t][p] : -1;
                 } else {
                     n.arg = flat[a];
+                    n.is_const = true;
                 }
             }
         } else {
@@ -961,6 +970,8 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
             }
             n.n_in = g.n_in;
             for (int i = 0; i < g.n_in; ++i) n.in[i] = stack[g.in[i]][base[g.in[i]]++];
+            n.is_const = true;
+            for (int i = 0; i < g.n_in; ++i) n.is_const = n.is_const && nodes[n.in[i]].is_const;
             for (int t = 0; t < N_STACKS; ++t) sp[t] -= cnt[t];
             n.out = g.out;
         }
@@ -1045,19 +1056,67 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
 
     // ---- accumulator form
     if ((forms & FORM_ACC) && root >= 0 && !has_stale_live && n_params < (1u << kLdOffsetBits)) {
+        // constant subtrees first: each a store behind the program's own
+        // constants, its node from then on a load of them
+        std::vector<int> &hoist = tls.hoist;
+        std::vector<Node> &kept = tls.hoisted_nodes;
+        hoist.clear();
+        kept.clear();
+        uint32_t types = 0, n_hoist = 0;
+        bool ok = true;
+        if (forms & FORM_HOIST) {
+            // the largest constant subtrees: those a node that is not
+            // constant reads, and the whole program's
+            for (size_t i = 0; i < nodes.size(); ++i) {
+                const Node &n = nodes[i];
+                if (!live[i] || n.is_const) continue;
+                for (int k = 0; k < n.n_in; ++k)
+                    if (nodes[n.in[k]].is_const && !is_load(nodes[n.in[k]].opcode)) hoist.push_back(n.in[k]);
+            }
+            if (nodes[root].is_const && !is_load(nodes[root].opcode)) hoist.push_back(root);
+            for (int id : hoist) n_hoist += kStackWidth[nodes[id].out];
+            if (n_params + n_hoist >= (1u << kLdOffsetBits)) hoist.clear();
+            n_hoist = 0;
+        }
+        if (!hoist.empty()) {
+            AccEmitter em(nodes);
+            ok = em.analyze(root);
+            for (size_t h = 0; ok && h < hoist.size(); ++h) {
+                Node &n = nodes[hoist[h]];
+                em.gen(hoist[h]);
+                em.emit(kTapeKind[n.out], n_params + n_hoist);
+                kept.push_back(n);
+                n.opcode = const_load_of(n.out);
+                n.n_in = 0;
+                n.arg = n_params + n_hoist;
+                n_hoist += kStackWidth[n.out];
+            }
+            if (fuse) fuse_loads(&em.code);
+            em.emit(K_STOP, 0);
+            types = em.types_;
+            for (int t = 0; t < N_STACKS; ++t) E.depth_fast[t] = em.max_sp[t];
+            E.reg_code.assign(em.code.begin(), em.code.end());
+        }
         AccEmitter em(nodes);
-        if (em.analyze(root)) {
+        if (ok && em.analyze(root)) {
             em.gen(root);
             if (fuse) fuse_loads(&em.code);
+            types |= em.types_;
             bool fits = true;
             for (int t = 0; t < N_STACKS; ++t) {
-                E.depth_fast[t] = em.max_sp[t];
-                fits = fits && em.max_sp[t] <= kMaxAccStack;
+                E.depth_fast[t] = std::max(E.depth_fast[t], em.max_sp[t]);
+                fits = fits && E.depth_fast[t] <= kMaxAccStack;
             }
             for (int p = 0; fits && p < N_PROFILES; ++p)
-                if ((em.types_ & ~kProfileTypes[p]) == 0) { E.profile = p; break; }
-            if (E.profile >= 0) E.reg_code.assign(em.code.begin(), em.code.end());
+                if ((types & ~kProfileTypes[p]) == 0) { E.profile = p; break; }
+            if (E.profile >= 0) {
+                E.main_off = (uint32_t)E.reg_code.size();
+                E.n_hoist = n_hoist;
+                E.reg_code.insert(E.reg_code.end(), em.code.begin(), em.code.end());
+            }
         }
+        if (E.profile < 0) E.reg_code.clear();
+        for (size_t h = 0; h < kept.size(); ++h) nodes[hoist[h]] = kept[h];
     }
 
     // ---- register adjoint form

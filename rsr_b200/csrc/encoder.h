@@ -43,6 +43,8 @@ struct EncodedProgram {
     int profile = -1;                     // -1: register kernel not applicable
     int depth_fast[N_STACKS] = {0, 0, 0, 0, 0};
     std::vector<uint32_t> reg_code;
+    uint32_t main_off = 0;                // first word of the main program (FORM_HOIST: behind the prologue)
+    uint32_t n_hoist = 0;                 // floats the prologue adds to the constants
     // adjoint (slot form with one slot range per value, never reused)
     std::vector<uint32_t> tape_code;      // 2 header words + 5 words per live node
     uint32_t n_tape_val = 0, n_tape_adj = 0;  // scalar value / adjoint slots
@@ -70,7 +72,8 @@ struct EncodedProgram {
 // Validates and encodes.  num_features == 0 skips feature-range checks.
 // Returns 0 or an rsr_status code, with a message in *err.
 // Device forms to emit (validation and the analysis run for every call).
-enum EncodeForms : unsigned { FORM_SLOT = 1u, FORM_TAPE = 2u, FORM_ACC = 4u, FORM_ADJ = 8u, FORM_ALL = 15u };
+enum EncodeForms : unsigned { FORM_SLOT = 1u, FORM_TAPE = 2u, FORM_ACC = 4u, FORM_ADJ = 8u, FORM_ALL = 15u,
+                             FORM_HOIST = 16u /* FORM_ACC with constant subtrees hoisted (uops.h) */ };
 int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uint32_t n_consts,
                    const float *params, uint32_t n_params, uint32_t num_features, EncodedProgram *out,
                    std::string *err, bool fuse_loads = true, unsigned forms = FORM_ALL);

@@ -39,6 +39,18 @@ static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec k
 #define RSR_BLOCK_M2 RSR_C27(K_M2)   // 104..130
 #define RSR_BLOCK_M3 RSR_C27(K_M3)   // 136..162
 
+// A prologue's store (uops.h, hoisted constants): every lane holds the same
+// value, and writes it.
+template <int PROF, int P, int t>
+__device__ __forceinline__ void store_const(Acc<PROF, P> &a, const AccIO<P> &io, uint32_t off) {
+    if constexpr (((kProfileTypes[PROF] >> t) & 1u) != 0u) {
+        constexpr int W = kStackWidth[t];
+        const Vf<P> *A = acc_of<PROF, P, t>(a);
+#pragma unroll
+        for (int c = 0; c < W; ++c) sts_f32(io.consts + 4u * (off + c), A[c].v[0]);
+    }
+}
+
 // Runs one program (accumulator form, ended by a K_STOP word) on this lane's
 // P points; the result is left in A_F.  OMIT: handlers left out of the kernel
 // because no program of the launch needs them -- bit 0: the unary Float ops
@@ -53,9 +65,12 @@ static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec k
 #define RSR_RUN(CASES)                                                   \
     switch (w & 0xFFu) {                                                 \
         CASES                                                            \
+        RSR_STORES                                                       \
         case K_STOP: return;                                             \
         default: __builtin_unreachable();                                \
     }
+#define RSR_S(T) case kTapeKind[T]: store_const<PROF, P, (T)>(a, io, arg); handler_end<kTapeKind[T]>(); break;
+#define RSR_STORES RSR_S(SF) RSR_S(SV2) RSR_S(SV3) RSR_S(SM2) RSR_S(SM3)
 template <int PROF, int P, int OMIT>
 __device__ __forceinline__ void run_program(Acc<PROF, P> &a, const AccIO<P> &io, uint32_t code) {
     constexpr bool NU = (OMIT & 1) != 0, NM = (OMIT & 2) != 0;
@@ -80,6 +95,8 @@ __device__ __forceinline__ void run_program(Acc<PROF, P> &a, const AccIO<P> &io,
 }
 
 #undef RSR_RUN
+#undef RSR_STORES
+#undef RSR_S
 #undef RSR_BLOCK_F
 #undef RSR_BLOCK_F_NU
 #undef RSR_BLOCK_V3_NM
@@ -96,6 +113,8 @@ __device__ __forceinline__ void run_program(Acc<PROF, P> &a, const AccIO<P> &io,
 __host__ __device__ __forceinline__ uint32_t align4r(uint32_t v) { return (v + 3u) & ~3u; }
 
 constexpr uint32_t kMaxProgsPerWarp = 8;
+static_assert(kMaxProgsPerWarp <= kRegThreads / 32, "a warp for each program's prologue");
+constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 // Block-cooperative item loop.  All warps of a block run the same programs
 // (one work item) on different tiles of the item's chunk, so the SM's
@@ -130,8 +149,8 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
     const int nw = blockDim.x >> 5;
     uint32_t *scode = reinterpret_cast<uint32_t *>(smem);
     float *sconst = smem + align4r(a.smem_code_words);
-    // [g][2] code and constants of each program, [24] item, [25] its
-    // programs, [26..27] targets' byte distance from the features, [28..29]
+    // [g][3] main program, constants and prologue (kNone: none) of each
+    // program, [24] item, [25] its programs, [26..27] targets' byte distance from the features, [28..29]
     // points to count, [30] last tile, [31] first program
     uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + align4r(a.smem_const_floats));
     double *red = reinterpret_cast<double *>(meta + 32);                                  // [warp][g]
@@ -164,11 +183,12 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
             uint32_t coff = 0, koff = 0;
             for (uint32_t g = 0; g < G; ++g) {
                 const ProgDesc pd = a.progs[it.prog_begin + g];
-                meta[2 * g] = coff;
-                meta[2 * g + 1] = koff;
+                meta[3 * g] = coff + pd.n_slots;
+                meta[3 * g + 1] = koff;
+                meta[3 * g + 2] = pd.n_slots ? coff : kNone;
                 scode[coff + pd.uop_len] = K_STOP;
                 coff += pd.uop_len + 1;
-                koff += pd.n_consts;
+                koff += pd.n_consts + pd.n_tape;
             }
             *reinterpret_cast<int64_t *>(meta + 26) =
                 reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
@@ -178,11 +198,14 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
             meta[31] = it.prog_begin;
         }
         __syncthreads();
+        bool hoisted = false;
         for (uint32_t g = 0; g < G; ++g) {
             const ProgDesc pd = a.progs[it.prog_begin + g];
-            for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) scode[meta[2 * g] + i] = __ldg(a.code + pd.uop_off + i);
+            uint32_t *code = scode + (meta[3 * g] - pd.n_slots);
+            for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) code[i] = __ldg(a.code + pd.uop_off + i);
             for (uint32_t i = threadIdx.x; i < pd.n_consts; i += blockDim.x)
-                sconst[meta[2 * g + 1] + i] = __ldg(a.consts + pd.const_off + i);
+                sconst[meta[3 * g + 1] + i] = __ldg(a.consts + pd.const_off + i);
+            hoisted |= pd.n_slots != 0u;
             sacc[(g * 2) * 32 + lane] = 0.0f;
             sacc[(g * 2 + 1) * 32 + lane] = 0.0f;
         }
@@ -194,12 +217,23 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
         // (shared memory and L1): held in registers it would be live across
         // the interpreter, which has none to spare at three blocks an SM.
         const volatile uint32_t *vmeta = meta;
-        for (uint32_t tile = it.tile_begin + warp; tile < vmeta[30]; tile += nw) {
+        // The item's prologues come first, as tile kNone: warp g runs program
+        // g's (one call of the interpreter in the kernel), then the block
+        // goes on to the tiles.
+        uint32_t tile = hoisted ? kNone : it.tile_begin + warp;
+        for (;;) {
+            if (tile != kNone && tile >= vmeta[30]) break;
             io.xl = opaque(ds.x + ((uint64_t)tile * (32u * P) + lane_point<P>(lane, 0)));
-            for (uint32_t g = 0; g < vmeta[25]; ++g) {
-                if (a.active && !a.active[vmeta[31] + g]) continue;
-                io.consts = opaque(smem_addr(sconst + meta[2 * g + 1]));
-                run_program<PROF, P, OMIT>(acc, io, opaque(smem_addr(scode + meta[2 * g])));
+            for (uint32_t g = tile == kNone ? (uint32_t)warp : 0u; g < vmeta[25]; ++g) {
+                const uint32_t at = vmeta[3 * g + (tile == kNone ? 2u : 0u)];
+                if (at == kNone) break;  // no prologue
+                if (a.active && !a.active[vmeta[31] + g]) {
+                    if (tile == kNone) break;
+                    continue;
+                }
+                io.consts = opaque(smem_addr(sconst + vmeta[3 * g + 1]));
+                run_program<PROF, P, OMIT>(acc, io, opaque(smem_addr(scode + at)));
+                if (tile == kNone) break;
                 const Vf<P> pred = acc.F[0];
                 const int64_t y_off = *reinterpret_cast<const volatile int64_t *>(vmeta + 26);
                 const uint64_t n_eval = *reinterpret_cast<const volatile uint64_t *>(vmeta + 28);
@@ -239,6 +273,12 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
                     sacc[(g * 2) * 32 + lane] = k.s;
                     sacc[(g * 2 + 1) * 32 + lane] = k.c;
                 }
+            }
+            if (tile == kNone) {
+                __syncthreads();
+                tile = a.items[vmeta[24]].tile_begin + warp;
+            } else {
+                tile += nw;
             }
         }
         if (a.mode == MODE_MSE) {

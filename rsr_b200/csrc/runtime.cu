@@ -247,7 +247,8 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
             pop.param_off[i + 1] < pop.param_off[i])
             return fail(RSR_EINVAL, "population offsets decrease at " + std::to_string(i));
     const bool fuse = (ctx->opts.flags & RSR_OPT_NO_LOAD_FUSION) == 0;
-    const unsigned forms = gradient ? (FORM_TAPE | FORM_ADJ) : kernel == RSR_KERNEL_PLAIN ? FORM_SLOT : FORM_ACC;
+    const unsigned forms = gradient ? (FORM_TAPE | FORM_ADJ) : kernel == RSR_KERNEL_PLAIN ? FORM_SLOT
+                                    : FORM_ACC | FORM_HOIST;
     std::vector<EncodedProgram> &enc = scratch ? scratch->enc : ctx->enc_cache;
     std::vector<int> &erc = scratch ? scratch->rc : ctx->enc_rc;
     std::vector<std::string> &emsg = scratch ? scratch->msg : ctx->enc_msg;
@@ -351,7 +352,7 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
             // one block next to the program's own code and constants
             uint32_t depth[N_STACKS];
             for (int t = 0; t < N_STACKS; ++t) depth[t] = (uint32_t)enc[i].depth_fast[t];
-            const uint32_t cw = (uint32_t)enc[i].reg_code.size() + 1, cf = (uint32_t)enc[i].consts.size();
+            const uint32_t cw = (uint32_t)enc[i].reg_code.size() + 1, cf = (uint32_t)enc[i].consts.size() + enc[i].n_hoist;
             if (reg_smem_bytes(cw, cf, depth, 2, 1) > kRegSmemBudget / 2) {
                 path[i] = -1;
             } else {
@@ -432,6 +433,9 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
             uint32_t depth[N_STACKS];
             for (int t = 0; t < N_STACKS; ++t) depth[t] = (uint32_t)E.adj_depth[t];
             d.n_tape = adj_pack_depth(depth);
+        } else if (path[i] >= 0) {
+            d.n_slots = E.main_off;
+            d.n_tape = E.n_hoist;
         } else {
             d.n_tape = E.n_tape_val | (E.n_tape_adj << 16);
         }
@@ -494,7 +498,7 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
             uint32_t cw = 0, cf = 0, sl = 0, len_sum = 0;
             for (uint32_t q = j; q < k; ++q) {
                 cw += P.progs[q].uop_len + 1;
-                cf += P.progs[q].n_consts;
+                cf += P.progs[q].n_consts + (g.kind == 1 ? P.progs[q].n_tape : 0u);
                 sl = std::max(sl, g.kind == 2 ? P.progs[q].n_tape & 0xFFFFu : P.progs[q].n_slots);
                 if (g.kind == 2) g.adj_slots = std::max(g.adj_slots, P.progs[q].n_tape >> 16);
                 len_sum += P.progs[q].uop_len;
@@ -1556,6 +1560,12 @@ int rsr_program_encoding(const rsr_program *prog, uint32_t num_features, int for
         v = {E.adj_profile < 0 ? 0xFFFFFFFFu : (uint32_t)E.adj_profile, E.adj_tape};
         for (int t = 0; t < N_STACKS; ++t) v.push_back((uint32_t)E.adj_depth[t]);
         v.insert(v.end(), E.adj_code.begin(), E.adj_code.end());
+    } else if (form == 6) {
+        if ((rc = encode_program(prog->code, prog->len, prog->const_kinds, prog->n_consts, prog->params,
+                                 prog->n_params, num_features, &E, &err, true, FORM_ACC | FORM_HOIST)))
+            return fail(rc, err);
+        v = {E.profile < 0 ? 0xFFFFFFFFu : (uint32_t)E.profile, E.main_off, E.n_hoist};
+        v.insert(v.end(), E.reg_code.begin(), E.reg_code.end());
     } else if (form == 4) {
         v.resize(noalloc_max_words());
         uint32_t nw = 0, ns = 0, fl = 0;

@@ -97,6 +97,15 @@ RSR_HD static constexpr int kv_make(int nbin, int w) { return kv_mulm(nbin, w) +
 
 RSR_HD static inline constexpr uint32_t uop_word(uint32_t kind, uint32_t arg) { return (kind & 0xFFu) | (arg << 8); }
 
+// Hoisted constants.  A subtree whose leaves are all constants has one value
+// for every point.  With FORM_HOIST such subtrees (the largest ones) become a
+// prologue, run once per work item instead of once per tile: the register
+// kernel's code is [prologue, K_STOP,] main program; a TAPE kind in the
+// prologue stores its type's accumulator to the constants, behind the
+// program's own (arg: flat offset), where the main program reads it.  The
+// values are those of the same micro-ops, so results do not change, and
+// constants that a fit rewrites between evaluations are folded afresh.
+
 // Fused loads.  A unary op (F unary, NORM/GET, DET/TRACE/TRANSPOSE/INVERSE)
 // may first load its operand, and a PUSH may be followed by a load:
 //   unary arg:  bits 0-11 feature or param offset, bits 12-13 load first
@@ -155,12 +164,12 @@ struct ProgDesc {
     uint32_t uop_len;     // words (slot form: 3 per instruction)
     uint32_t const_off;   // first float in the launch's constant pool
     uint32_t n_consts;    // floats
-    uint32_t n_slots;     // slot form: scalar slots needed
+    uint32_t n_slots;     // slot form: scalar slots needed; accumulator form: first word of the main program
     uint32_t flags;       // PF_* below
     uint32_t dataset;     // index into the launch's dataset table
     uint32_t part_off;    // first partial-sum slot of this program
     uint32_t n_parts;     // partial-sum slots (chunks) of this program
-    uint32_t n_tape;      // adjoint kernel: value slots | adjoint slots << 16
+    uint32_t n_tape;      // adjoint kernel: value slots | adjoint slots << 16; accumulator form: hoisted floats
 };
 enum : uint32_t { PF_RESULT_ZERO = 1u, PF_NEEDS_ZERO_INIT = 2u, PF_DIFFERENTIABLE = 4u };
 
