@@ -87,42 +87,47 @@ TaskPool::~TaskPool() {
     for (auto &t : threads_) t.join();
 }
 
-void TaskPool::work() {
-    uint64_t seen = 0;
-    for (;;) {
-        const std::function<void(uint32_t)> *f;
-        uint32_t n;
-        {
-            std::unique_lock<std::mutex> lk(mu_);
-            cv_.wait(lk, [&] { return stop_ || epoch_ != seen; });
-            if (stop_) return;
-            seen = epoch_;
-            f = task_;
-            n = n_;
-        }
-        for (uint32_t i = next_.fetch_add(1); i < n; i = next_.fetch_add(1)) (*f)(i);
-        {
+void TaskPool::help(Job &j) {
+    for (uint32_t i = j.next.fetch_add(1); i < j.n; i = j.next.fetch_add(1)) {
+        j.f(i);
+        if (j.done.fetch_add(1, std::memory_order_acq_rel) + 1 == j.n) {
             std::lock_guard<std::mutex> lk(mu_);
-            if (++finished_ == threads_.size()) done_cv_.notify_all();
+            done_cv_.notify_all();
         }
     }
 }
 
-void TaskPool::run(uint32_t n, const std::function<void(uint32_t)> &f) {
+void TaskPool::work() {
+    std::shared_ptr<Job> job;
+    for (;;) {
+        {
+            std::unique_lock<std::mutex> lk(mu_);
+            cv_.wait(lk, [&] { return stop_ || job_ != job; });
+            if (stop_) return;
+            job = job_;
+        }
+        if (job) help(*job);
+    }
+}
+
+void TaskPool::begin(uint32_t n, std::function<void(uint32_t)> f) {
     {
         std::lock_guard<std::mutex> lk(mu_);
-        task_ = &f;
-        n_ = n;
-        next_.store(0);
-        finished_ = 0;
-        ++epoch_;
+        job_ = std::make_shared<Job>();
+        job_->f = std::move(f);
+        job_->n = n;
     }
     cv_.notify_all();
-    for (uint32_t i = next_.fetch_add(1); i < n; i = next_.fetch_add(1)) f(i);
-    // every worker takes part in every run and has left it before the next
-    // one starts, so none can pick up this run's task or counter late
+}
+
+void TaskPool::end() {
+    // a worker that wakes late finds its job's counter used up: it calls
+    // nothing, so what the tasks refer to may go once all of them are done
+    const std::shared_ptr<Job> j = job_;
+    if (!j) return;
+    help(*j);
     std::unique_lock<std::mutex> lk(mu_);
-    done_cv_.wait(lk, [&] { return finished_ == threads_.size(); });
+    done_cv_.wait(lk, [&] { return j->done.load(std::memory_order_acquire) == j->n; });
 }
 
 // register path = profile + 8 * (spill-depth class + 3 * omitted-handler mask)
@@ -203,202 +208,243 @@ static TuneChoice choice_for(rsr_ctx *ctx, int profile, uint64_t n_eval) {
     return c;
 }
 
-int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_prog, uint64_t ds_all, int kernel,
-               bool gradient, int mode, Plan *plan, EncodeScratch *scratch, std::mutex *table_mu) {
-    NvtxRange nvtx_range("rsr: encode + plan");
+// The register adjoint's launch for a program: the most points per lane (8,
+// 4, 2) whose tape fits a warp's share of the SM's tensor memory (512 columns /
+// (warps / 4), P columns a slot) and whose stacks and sums fit the block's
+// shared memory; launches by points per lane and profile.  -1: the slot-file
+// adjoint.  omit: the handler sets the program does not use (forward entries:
+// two words each after the header words); a launch leaves out those none of its
+// programs uses.
+static int adjoint_path(const EncodedProgram &E, uint8_t *omit_out) {
+    if (E.adj_profile < 0 || !adj_supported(E.adj_profile)) return -1;
+    uint32_t depth[N_STACKS];
+    for (int t = 0; t < N_STACKS; ++t) depth[t] = (uint32_t)E.adj_depth[t];
+    const uint32_t np = (uint32_t)E.consts.size();
+    int pc = adj_max_p(E.adj_profile) >= 8 ? 2 : 1;  // points per lane 2 << pc
+    for (; pc >= 0; --pc) {
+        const int P = 2 << pc, nw = adj_block_warps(E.adj_profile, P);
+        const uint32_t cols = 512u / (uint32_t)(nw / 4);
+        if (E.adj_tape * (uint32_t)P <= cols &&
+            (size_t)adj_warp_floats(depth, P, np) * 4u * (size_t)nw <= kAdjRegionBudget)
+            break;
+    }
+    if (pc < 0) return -1;
+    const uint32_t mv = (uint32_t)(K_V3 + kv_mulm(kBinOps[SV3], 3));
+    unsigned omit = adj_omittable(E.adj_profile);
+    const uint32_t n_fwd = E.adj_code.empty() ? 0u : E.adj_code[0];
+    for (uint32_t q = 0; q < n_fwd; ++q) {
+        const uint32_t kind = E.adj_code[kAdjHeaderWords + 2 * q] & 0xFFu;
+        if (kind >= (uint32_t)K_F_UN && kind < (uint32_t)K_F_END) omit &= ~1u;
+        if (kind >= mv + 1 && kind <= mv + 3) omit &= ~2u;
+    }
+    *omit_out = (uint8_t)omit;
+    return kAdjPathBase + pc * N_PROFILES + E.adj_profile;
+}
+
+// The slot-file adjoint's launch for a program (<= -2): by tape size, so that
+// a block's shared memory follows its own programs' tapes: steps of 16 slots
+// up to 256, then <= 512 and more (a launch sizes every warp's tape for its
+// largest program, and a finer step packs more tapes per SM).
+static int slot_adjoint_path(const EncodedProgram &E) {
+    const uint32_t nt = E.n_tape_val + E.n_tape_adj;
+    const int bucket = nt <= 256 ? (int)((nt + 15) / 16) : nt <= 512 ? 17 : 18;
+    // Points per lane: the most (4, 2, 1) whose tape fits kGradTapeBudget,
+    // decided from the program alone, so that its sums do not depend on the
+    // other programs of the call.
+    int lp = 2;
+    while (lp > 0 && grad_smem_per_warp((uint32_t)E.tape_code.size() + 1, (uint32_t)E.consts.size(), E.n_tape_val,
+                                        E.n_tape_adj, 1 << lp) > kGradTapeBudget)
+        --lp;
+    // programs without a unary Float op run on a kernel built without those
+    // handlers (F and F+V3 profiles)
+    bool nu = grad_has_no_unary(E.tape_profile);
+    for (size_t w = 2; w + 5 <= E.tape_code.size(); w += 5) {
+        const uint32_t op = E.tape_code[w] & 0xFFu;
+        if (op >= (uint32_t)SIN_F && op <= (uint32_t)LN_F) nu = false;
+    }
+    // one launch per (tape-size bucket, points per lane, no-unary flag, kernel profile)
+    return -2 - (((bucket * 3 + lp) * 2 + (nu ? 1 : 0)) * N_PROFILES + E.tape_profile);
+}
+
+// The register kernel's launch for a program, -1 if it needs the slot-file kernel.
+static int register_path(const EncodedProgram &E) {
+    if (E.profile < 0) return -1;
+    // the spill stacks for 2 points per lane must fit one block next to the
+    // program's own code and constants
+    uint32_t depth[N_STACKS];
+    for (int t = 0; t < N_STACKS; ++t) depth[t] = (uint32_t)E.depth_fast[t];
+    const uint32_t cw = (uint32_t)E.reg_code.size() + 1, cf = (uint32_t)E.consts.size() + E.n_hoist;
+    if (reg_smem_bytes(cw, cf, depth, 2, 1) > kRegSmemBudget / 2) return -1;
+    // launches by spill depth, so that shallow programs (most of a random
+    // population) run with small spill stacks and leave the SM's unified L1
+    // to their feature loads
+    uint32_t dmax = 0;
+    for (int t = 0; t < N_STACKS; ++t) dmax = std::max(dmax, depth[t]);
+    const int cls = dmax <= 1 ? 0 : dmax <= 2 ? 1 : 2;
+    // and apart by the handler sets the program does not use (unary Float
+    // ops; mat-vec with a leaf or spilled matrix), whose kernels are built
+    // without them: smaller kernels, fewer instruction-cache misses
+    const uint32_t mv = (uint32_t)(K_V3 + kv_mulm(kBinOps[SV3], 3));
+    unsigned omit = reg_omittable(E.profile);
+    for (uint32_t w : E.reg_code) {
+        const uint32_t kind = w & 0xFFu;
+        if (kind >= (uint32_t)K_F_UN && kind < (uint32_t)K_F_END) omit &= ~1u;
+        if (kind >= mv + 1 && kind <= mv + 3) omit &= ~2u;
+    }
+    return E.profile + kRegPathStride * (cls + 3 * (int)omit);
+}
+
+// Stable sort by key: bytes that are the same in all keys are skipped, so a
+// population's keys (few paths and datasets, code lengths below 256) take
+// three or four counting passes.
+static void sort_by_key(std::vector<std::pair<uint64_t, uint32_t>> *v, std::vector<std::pair<uint64_t, uint32_t>> *tmp) {
+    uint64_t differ = 0;
+    for (const auto &e : *v) differ |= e.first ^ (*v)[0].first;
+    tmp->resize(v->size());
+    for (int sh = 0; sh < 64; sh += 8) {
+        if (!((differ >> sh) & 0xFFu)) continue;
+        uint32_t at[257] = {0};
+        for (const auto &e : *v) at[((e.first >> sh) & 0xFFu) + 1]++;
+        for (int b = 0; b < 256; ++b) at[b + 1] += at[b];
+        for (const auto &e : *v) (*tmp)[at[(e.first >> sh) & 0xFFu]++] = e;
+        v->swap(*tmp);
+    }
+}
+
+// Planning in two halves.  begin_plan looks the datasets up and starts
+// encoding the programs, each only in the form its kernel needs, on the
+// encoding threads; end_plan waits for them and lays the launch out.  Between
+// the two the caller may end another plan: a chunked call lays chunk k out
+// while the threads encode chunk k + 1.
+static TaskPool *pool_of(rsr_ctx *ctx, EncodeScratch *S) {
+    std::unique_ptr<TaskPool> &pool = S->shared_pool ? ctx->encoders : S->pool;
+    if (!pool)
+        pool = std::make_unique<TaskPool>(std::max(1u, std::min(S->threads, std::thread::hardware_concurrency())));
+    return pool.get();
+}
+
+static int begin_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_prog, uint64_t ds_all, int kernel,
+                      bool gradient, int mode, Plan *plan, EncodeScratch *S, std::mutex *table_mu) {
+    NvtxRange nvtx_range("rsr: encode");
     Plan &P = *plan;
     P.reset();
     P.gradient = gradient;
     P.mode = mode;
     const uint32_t n = pop.n_programs;
+    S->running = false;
     if (n == 0) return RSR_OK;
     if (!pop.code_off || !pop.kind_off || !pop.param_off) return fail(RSR_EINVAL, "population offsets are null");
-    // The first gradient plan of a context loads every kernel instance (the
-    // caller holds ctx->mu here), ~40 ms: a 20-iteration fit of the matrix
-    // workload whose adjoint instances were first launched from its
-    // captured iteration took 0.95 s, 0.22 s once they had been launched.
-    if (gradient && !scratch && !ctx->kernels_loaded) {
-        const int rc = preload_eval_kernels(ctx);
-        if (rc) return rc;
-    }
     // datasets
-    std::map<uint64_t, uint32_t> ds_index;
-    std::vector<uint32_t> prog_ds(n);
-    std::unique_lock<std::mutex> table_lock;
-    if (table_mu) table_lock = std::unique_lock<std::mutex>(*table_mu);
-    for (uint32_t i = 0; i < n; ++i) {
-        uint64_t h = ds_per_prog ? ds_per_prog[i] : ds_all;
-        auto f = ds_index.find(h);
-        if (f == ds_index.end()) {
-            auto it = ctx->datasets.find(h);
-            if (it == ctx->datasets.end()) return fail(RSR_ENOTFOUND, "unknown dataset handle " + std::to_string(h));
-            uint32_t idx = (uint32_t)P.datasets.size();
-            P.datasets.push_back(it->second->desc());
-            P.ds_handles.push_back(h);
-            f = ds_index.emplace(h, idx).first;
+    S->prog_ds.resize(n);
+    {
+        std::unique_lock<std::mutex> table_lock;
+        if (table_mu) table_lock = std::unique_lock<std::mutex>(*table_mu);
+        std::map<uint64_t, uint32_t> ds_index;
+        uint64_t last = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            const uint64_t h = ds_per_prog ? ds_per_prog[i] : ds_all;
+            if (i > 0 && h == last) {
+                S->prog_ds[i] = S->prog_ds[i - 1];
+                continue;
+            }
+            auto f = ds_index.find(h);
+            if (f == ds_index.end()) {
+                auto it = ctx->datasets.find(h);
+                if (it == ctx->datasets.end()) return fail(RSR_ENOTFOUND, "unknown dataset handle " + std::to_string(h));
+                f = ds_index.emplace(h, (uint32_t)P.datasets.size()).first;
+                P.datasets.push_back(it->second->desc());
+                P.ds_handles.push_back(h);
+            }
+            S->prog_ds[i] = f->second;
+            last = h;
         }
-        prog_ds[i] = f->second;
     }
-    if (table_lock.owns_lock()) table_lock.unlock();
-    // encode: each program only in the form its kernel needs, in parallel
-    // for large populations
     for (uint32_t i = 0; i < n; ++i)
         if (pop.code_off[i + 1] < pop.code_off[i] || pop.kind_off[i + 1] < pop.kind_off[i] ||
             pop.param_off[i + 1] < pop.param_off[i])
             return fail(RSR_EINVAL, "population offsets decrease at " + std::to_string(i));
+    if (S->enc.size() < n) {
+        S->enc.resize(n);
+        S->rc.resize(n);
+        S->msg.resize(n);
+    }
+    S->path.assign(n, 0);
+    S->adj_omit.assign(n, 0);
     const bool fuse = (ctx->opts.flags & RSR_OPT_NO_LOAD_FUSION) == 0;
-    const unsigned forms = gradient ? (FORM_TAPE | FORM_ADJ) : kernel == RSR_KERNEL_PLAIN ? FORM_SLOT
-                                    : FORM_ACC | FORM_HOIST;
-    std::vector<EncodedProgram> &enc = scratch ? scratch->enc : ctx->enc_cache;
-    std::vector<int> &erc = scratch ? scratch->rc : ctx->enc_rc;
-    std::vector<std::string> &emsg = scratch ? scratch->msg : ctx->enc_msg;
-    if (enc.size() < n) {
-        enc.resize(n);
-        erc.resize(n);
-        emsg.resize(n);
-    }
-    auto encode_one = [&](uint32_t i, unsigned f) {
-        const uint64_t c0 = pop.code_off[i], k0 = pop.kind_off[i], p0 = pop.param_off[i];
-        erc[i] = encode_program(pop.code + c0, (uint32_t)(pop.code_off[i + 1] - c0), pop.const_kinds + k0,
-                                (uint32_t)(pop.kind_off[i + 1] - k0), pop.params + p0,
-                                (uint32_t)(pop.param_off[i + 1] - p0), P.datasets[prog_ds[i]].num_features, &enc[i],
-                                &emsg[i], fuse, f);
-    };
-    if (n >= 64) {  // a program takes ~2 us to encode; a pool run costs ~10 us
-        std::unique_ptr<TaskPool> &pool = scratch ? scratch->pool : ctx->encoders;
-        if (!pool)
-            pool = std::make_unique<TaskPool>(std::max(
-                1u, std::min(scratch ? scratch->threads : 16u, std::thread::hardware_concurrency())));
-        // programs in blocks of 16 per task
-        const uint32_t nb = (n + 15) / 16;
-        pool->run(nb, [&](uint32_t b) {
-            for (uint32_t i = b * 16; i < std::min(n, b * 16 + 16); ++i) encode_one(i, forms);
-        });
-    } else {
-        for (uint32_t i = 0; i < n; ++i) encode_one(i, forms);
-    }
-    for (uint32_t i = 0; i < n; ++i)
-        if (erc[i] != RSR_OK) return fail(erc[i], "program " + std::to_string(i) + ": " + emsg[i]);
+    const unsigned forms = gradient ? (ctx->opts.flags & RSR_OPT_SLOT_ADJOINT ? FORM_TAPE : FORM_ADJ)
+                         : kernel == RSR_KERNEL_PLAIN ? FORM_SLOT : FORM_ACC | FORM_HOIST;
+    const std::vector<DatasetDesc> *datasets = &P.datasets;
     // path per program: <= -2 slot-file adjoint, -1 plain, >= 0 register
     // profile (MSE plans) or register adjoint (gradient plans)
-    std::vector<int> path(n);
-    std::vector<uint8_t> adj_omit(n, 0);
-    for (uint32_t i = 0; i < n; ++i) {
-        if (gradient && enc[i].adj_profile >= 0 && adj_supported(enc[i].adj_profile) &&
-            !(ctx->opts.flags & RSR_OPT_SLOT_ADJOINT)) {
-            // register adjoint: the most points per lane (8, 4, 2) whose tape
-            // fits a warp's share of the SM's tensor memory (512 columns / (warps
-            // / 4), P columns a slot) and whose stacks and sums fit the block's
-            // shared memory; launches by points per lane and profile
-            const EncodedProgram &E = enc[i];
-            uint32_t depth[N_STACKS];
-            for (int t = 0; t < N_STACKS; ++t) depth[t] = (uint32_t)E.adj_depth[t];
-            const uint32_t np = (uint32_t)E.consts.size();
-            int pc = adj_max_p(E.adj_profile) >= 8 ? 2 : 1;  // points per lane 2 << pc
-            for (; pc >= 0; --pc) {
-                const int P = 2 << pc, nw = adj_block_warps(E.adj_profile, P);
-                const uint32_t cols = 512u / (uint32_t)(nw / 4);
-                if (E.adj_tape * (uint32_t)P <= cols &&
-                    (size_t)adj_warp_floats(depth, P, np) * 4u * (size_t)nw <= kAdjRegionBudget)
-                    break;
-            }
-            if (pc >= 0) {
-                const int bucket = 0;
-                // the handler sets the program does not use (forward entries:
-                // two words each after the header words); a launch leaves out
-                // those none of its programs uses
-                const uint32_t mv = (uint32_t)(K_V3 + kv_mulm(kBinOps[SV3], 3));
-                unsigned omit = adj_omittable(E.adj_profile);
-                const uint32_t n_fwd = E.adj_code.empty() ? 0u : E.adj_code[0];
-                for (uint32_t q = 0; q < n_fwd; ++q) {
-                    const uint32_t kind = E.adj_code[kAdjHeaderWords + 2 * q] & 0xFFu;
-                    if (kind >= (uint32_t)K_F_UN && kind < (uint32_t)K_F_END) omit &= ~1u;
-                    if (kind >= mv + 1 && kind <= mv + 3) omit &= ~2u;
-                }
-                adj_omit[i] = (uint8_t)omit;
-                path[i] = kAdjPathBase + ((bucket * 3 + pc) * N_PROFILES + E.adj_profile);
-                continue;
-            }
+    auto one = [S, pop, datasets, fuse, forms, gradient](uint32_t i) {
+        EncodedProgram &E = S->enc[i];
+        auto encode = [&](unsigned f) {
+            const uint64_t c0 = pop.code_off[i], k0 = pop.kind_off[i], p0 = pop.param_off[i];
+            S->rc[i] = encode_program(pop.code + c0, (uint32_t)(pop.code_off[i + 1] - c0), pop.const_kinds + k0,
+                                      (uint32_t)(pop.kind_off[i + 1] - k0), pop.params + p0,
+                                      (uint32_t)(pop.param_off[i + 1] - p0), (*datasets)[S->prog_ds[i]].num_features,
+                                      &E, &S->msg[i], fuse, f);
+            return S->rc[i] == RSR_OK;
+        };
+        if (!encode(forms)) return;
+        int path = forms & FORM_ADJ ? adjoint_path(E, &S->adj_omit[i]) : forms & FORM_ACC ? register_path(E) : -1;
+        if (gradient && path < 0) {
+            if (!(forms & FORM_TAPE) && !encode(FORM_TAPE)) return;
+            path = slot_adjoint_path(E);
+        } else if (path < 0 && !(forms & FORM_SLOT) && !encode(FORM_SLOT)) {
+            return;  // programs the register kernel cannot take run on the slot-file kernel
         }
-        if (gradient) {
-            // adjoint launches by tape size, so that a block's shared memory
-            // follows its own programs' tapes: steps of 16 slots up to 256,
-            // then <= 512 and more (a launch sizes every warp's tape for its
-            // largest program, and a finer step packs more tapes per SM)
-            const uint32_t nt = enc[i].n_tape_val + enc[i].n_tape_adj;
-            const int bucket = nt <= 256 ? (int)((nt + 15) / 16) : nt <= 512 ? 17 : 18;
-            // Points per lane: the most (4, 2, 1) whose tape fits
-            // kGradTapeBudget, decided from the program alone, so that its
-            // sums do not depend on the other programs of the call.
-            int lp = 2;
-            while (lp > 0 && grad_smem_per_warp((uint32_t)enc[i].tape_code.size() + 1, (uint32_t)enc[i].consts.size(),
-                                                enc[i].n_tape_val, enc[i].n_tape_adj, 1 << lp) > kGradTapeBudget)
-                --lp;
-            // programs without a unary Float op run on a kernel built without
-            // those handlers (F and F+V3 profiles)
-            bool nu = grad_has_no_unary(enc[i].tape_profile);
-            const std::vector<uint32_t> &tc = enc[i].tape_code;
-            for (size_t w = 2; w + 5 <= tc.size(); w += 5) {
-                const uint32_t op = tc[w] & 0xFFu;
-                if (op >= (uint32_t)SIN_F && op <= (uint32_t)LN_F) nu = false;
-            }
-            // one launch per (tape-size bucket, points per lane, no-unary
-            // flag, kernel profile)
-            path[i] = -2 - (((bucket * 3 + lp) * 2 + (nu ? 1 : 0)) * N_PROFILES + enc[i].tape_profile);
-        }
-        else if (kernel == RSR_KERNEL_PLAIN || enc[i].profile < 0) path[i] = -1;
-        else {
-            // the register kernel's spill stacks for 2 points per lane must fit
-            // one block next to the program's own code and constants
-            uint32_t depth[N_STACKS];
-            for (int t = 0; t < N_STACKS; ++t) depth[t] = (uint32_t)enc[i].depth_fast[t];
-            const uint32_t cw = (uint32_t)enc[i].reg_code.size() + 1, cf = (uint32_t)enc[i].consts.size() + enc[i].n_hoist;
-            if (reg_smem_bytes(cw, cf, depth, 2, 1) > kRegSmemBudget / 2) {
-                path[i] = -1;
-            } else {
-                // launches by spill depth, so that shallow programs (most of
-                // a random population) run with small spill stacks and leave
-                // the SM's unified L1 to their feature loads
-                uint32_t dmax = 0;
-                for (int t = 0; t < N_STACKS; ++t) dmax = std::max(dmax, depth[t]);
-                const int cls = dmax <= 1 ? 0 : dmax <= 2 ? 1 : 2;
-                // and apart by the handler sets the program does not use
-                // (unary Float ops; mat-vec with a leaf or spilled matrix),
-                // whose kernels are built without them: smaller kernels,
-                // fewer instruction-cache misses
-                const uint32_t mv = (uint32_t)(K_V3 + kv_mulm(kBinOps[SV3], 3));
-                unsigned omit = reg_omittable(enc[i].profile);
-                for (uint32_t w : enc[i].reg_code) {
-                    const uint32_t kind = w & 0xFFu;
-                    if (kind >= (uint32_t)K_F_UN && kind < (uint32_t)K_F_END) omit &= ~1u;
-                    if (kind >= mv + 1 && kind <= mv + 3) omit &= ~2u;
-                }
-                path[i] = enc[i].profile + kRegPathStride * (cls + 3 * (int)omit);
-            }
-        }
-        // programs the register kernel cannot take run on the slot-file kernel
-        if (path[i] == -1 && !(forms & FORM_SLOT)) {
-            encode_one(i, FORM_SLOT);
-            if (erc[i] != RSR_OK) return fail(erc[i], "program " + std::to_string(i) + ": " + emsg[i]);
-        }
+        S->path[i] = path;
+    };
+    if (n >= 64) {  // a program takes ~2 us to encode; starting the threads costs ~10 us
+        // programs in blocks of 16 per task
+        pool_of(ctx, S)->begin((n + 15) / 16, [one, n](uint32_t b) {
+            for (uint32_t i = b * 16; i < std::min(n, b * 16 + 16); ++i) one(i);
+        });
+        S->running = true;
+    } else {
+        for (uint32_t i = 0; i < n; ++i) one(i);
     }
+    return RSR_OK;
+}
+
+// Waits for the encoding that begin_plan started (also before giving up on it).
+static void wait_plan(rsr_ctx *ctx, EncodeScratch *S) {
+    if (S->running) pool_of(ctx, S)->end();
+    S->running = false;
+}
+
+static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeScratch *S, std::mutex *table_mu) {
+    NvtxRange nvtx_range("rsr: plan");
+    Plan &P = *plan;
+    const bool gradient = P.gradient;
+    const uint32_t n = pop.n_programs;
+    if (n == 0) return RSR_OK;
+    const std::vector<EncodedProgram> &enc = S->enc;
+    const std::vector<int> &path = S->path;
+    const std::vector<uint8_t> &adj_omit = S->adj_omit;
+    const std::vector<uint32_t> &prog_ds = S->prog_ds;
+    for (uint32_t i = 0; i < n; ++i)
+        if (S->rc[i] != RSR_OK) return fail(S->rc[i], "program " + std::to_string(i) + ": " + S->msg[i]);
+    std::unique_lock<std::mutex> table_lock;
     // group programs by (path, dataset), each group sorted by descending code length
     // (one 64-bit key per program: path, dataset, then longer code first and
     // the caller's order among equals, as a stable sort by those would give)
-    std::vector<uint32_t> order(n);
+    std::vector<uint32_t> &order = P.orig;
+    order.resize(n);
     {
-        std::vector<std::pair<uint64_t, uint32_t>> keyed(n);
+        static thread_local std::vector<std::pair<uint64_t, uint32_t>> keyed, spare;
+        keyed.resize(n);
         for (uint32_t i = 0; i < n; ++i) {
             const uint64_t len = enc[i].reg_code.size() + enc[i].slot_code.size();
             const uint64_t key = ((uint64_t)(uint32_t)(path[i] + (1 << 20)) << 42) | ((uint64_t)prog_ds[i] << 22) |
                                  ((1ull << 22) - 1 - std::min<uint64_t>(len, (1ull << 22) - 1));
             keyed[i] = {key, i};
         }
-        std::sort(keyed.begin(), keyed.end());
+        sort_by_key(&keyed, &spare);
         for (uint32_t i = 0; i < n; ++i) order[i] = keyed[i].second;
     }
     P.progs.resize(n);
-    P.orig = order;
     {
         size_t cw = 0, cf = 0;
         for (uint32_t i = 0; i < n; ++i) {
@@ -554,14 +600,16 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
         std::stable_sort(items.begin(), items.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
         full.clear();
         tail.clear();
+        auto tiles_of = [&](const WorkItem &w) {
+            return (P.datasets[P.progs[w.prog_begin].dataset].n_eval + tile_pts - 1) / tile_pts;
+        };
         for (auto &pr : items) {
             const WorkItem &w = pr.second;
-            const uint64_t n_eval = P.datasets[P.progs[w.prog_begin].dataset].n_eval;
-            const uint64_t n_tiles = (n_eval + tile_pts - 1) / tile_pts;
+            const uint64_t n_tiles = tiles_of(w);
+            WorkItem it = w;
             if (g.kind == 3) {  // parts spread evenly over the items
                 const uint64_t n_parts = P.progs[w.prog_begin].n_parts, m = n_tiles ? adj_items(n_parts, g.parts) : 0;
                 for (uint64_t c = 0; c < m; ++c) {
-                    WorkItem it = w;
                     const uint64_t p0 = c * n_parts / m, p1 = (c + 1) * n_parts / m;
                     it.tile_begin = (uint32_t)(p0 * part_tiles);
                     it.tile_end = (uint32_t)std::min(n_tiles, p1 * part_tiles);
@@ -569,23 +617,41 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
                     const uint64_t tiles = it.tile_end - it.tile_begin;
                     (tiles == tpc ? full : tail).emplace_back(pr.first * tiles, it);
                 }
-                continue;
-            }
-            for (uint64_t c = 0, t = 0; t < n_tiles; ++c, t += tpc) {
-                WorkItem it = w;
-                it.tile_begin = (uint32_t)t;
-                it.tile_end = (uint32_t)std::min(n_tiles, t + tpc);
-                it.chunk = (uint32_t)c;
-                const uint64_t tiles = it.tile_end - it.tile_begin;
-                (tiles == tpc ? full : tail).emplace_back(pr.first * tiles, it);
+            } else if (n_tiles % tpc) {
+                it.chunk = (uint32_t)(n_tiles / tpc);
+                it.tile_begin = (uint32_t)(it.chunk * tpc);
+                it.tile_end = (uint32_t)n_tiles;
+                tail.emplace_back(pr.first * (n_tiles % tpc), it);
             }
         }
         std::stable_sort(tail.begin(), tail.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
-        g.item_work = std::max(full.empty() ? 0 : full[0].first, tail.empty() ? 0 : tail[0].first);
-        size_t a = 0, b = 0;
-        while (a < full.size() || b < tail.size())
-            P.items.push_back(b == tail.size() || (a < full.size() && full[a].first >= tail[b].first) ? full[a++].second
-                                                                                                   : tail[b++].second);
+        size_t b = 0;
+        auto short_ones = [&](uint64_t longer_than) {
+            for (; b < tail.size() && tail[b].first > longer_than; ++b) P.items.push_back(tail[b].second);
+        };
+        if (g.kind == 3) {
+            g.item_work = std::max(full.empty() ? 0 : full[0].first, tail.empty() ? 0 : tail[0].first);
+            for (auto &f : full) {
+                short_ones(f.first);
+                P.items.push_back(f.second);
+            }
+        } else {
+            g.item_work = tail.empty() ? 0 : tail[0].first;
+            for (auto &pr : items) {  // the full chunks, generated where they go
+                const uint64_t n_full = tiles_of(pr.second) / tpc, work = pr.first * tpc;
+                if (n_full == 0) continue;
+                g.item_work = std::max(g.item_work, work);
+                short_ones(work);
+                WorkItem it = pr.second;
+                for (uint64_t c = 0; c < n_full; ++c) {
+                    it.tile_begin = (uint32_t)(c * tpc);
+                    it.tile_end = (uint32_t)((c + 1) * tpc);
+                    it.chunk = (uint32_t)c;
+                    P.items.push_back(it);
+                }
+            }
+        }
+        for (; b < tail.size(); ++b) P.items.push_back(tail[b].second);
         g.n_items = (uint32_t)P.items.size() - g.item_begin;
         for (uint32_t q = li; q < end; ++q) {
             const EncodedProgram &E = enc[order[q]];
@@ -601,6 +667,23 @@ int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_p
     std::stable_sort(P.groups.begin(), P.groups.end(),
                      [](const Group &a, const Group &b) { return a.item_work > b.item_work; });
     return RSR_OK;
+}
+
+int build_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *ds_per_prog, uint64_t ds_all, int kernel,
+               bool gradient, int mode, Plan *plan, EncodeScratch *scratch, std::mutex *table_mu) {
+    // The first gradient plan of a context loads every kernel instance (the
+    // caller holds ctx->mu here), ~40 ms: a 20-iteration fit of the matrix
+    // workload whose adjoint instances were first launched from its
+    // captured iteration took 0.95 s, 0.22 s once they had been launched.
+    if (gradient && !scratch && !ctx->kernels_loaded && pop.n_programs > 0) {
+        const int rc = preload_eval_kernels(ctx);
+        if (rc) return rc;
+    }
+    EncodeScratch *S = scratch ? scratch : &ctx->enc[0];
+    int rc = begin_plan(ctx, pop, ds_per_prog, ds_all, kernel, gradient, mode, plan, S, table_mu);
+    if (rc) return rc;
+    wait_plan(ctx, S);
+    return end_plan(ctx, pop, plan, S, table_mu);
 }
 
 int upload_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t st) {
@@ -883,8 +966,9 @@ static rsr_population single_pop(const rsr_program *p, uint64_t offs[6]) {
     return pop;
 }
 
-// A large MSE (or MSE + gradient) call in chunks of programs: the host
-// encodes chunk k+1 while the device runs chunk k.  Chunks alternate between
+// A large MSE (or MSE + gradient) call in chunks of programs: the encoding
+// threads encode chunk k+1 while this one lays chunk k out and the device
+// runs the chunks before it.  Chunks alternate between
 // two device plans, each with its own stream, so chunk k+1's first launch
 // fills the SMs that chunk k's last blocks leave; a plan's buffers are
 // rewritten by a later chunk on the same stream, after the device is done
@@ -905,35 +989,60 @@ static int run_chunked(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *
         cudaStreamSynchronize(ctx->stream);
     };
     uint64_t h2d = 0;
+    if (gradient && !ctx->kernels_loaded) {
+        const int rc = preload_eval_kernels(ctx);
+        if (rc) return rc;
+    }
+    auto part_of = [&](uint32_t k) {
+        rsr_population sub = pop;
+        sub.n_programs = start[k + 1] - start[k];
+        sub.code_off = pop.code_off + start[k];
+        sub.kind_off = pop.kind_off + start[k];
+        sub.param_off = pop.param_off + start[k];
+        return sub;
+    };
+    auto begin = [&](uint32_t k) {
+        return begin_plan(ctx, part_of(k), dsp ? dsp + start[k] : nullptr, ds, kernel, gradient, MODE_MSE, &plans[k],
+                          &ctx->enc[k & 1], nullptr);
+    };
+    // reports a program by its index in the caller's population
+    auto plan_fail = [&](int rc, uint32_t k) {
+        std::string m = rsr_last_error();
+        const size_t at = m.rfind("program ", 0) == 0 ? 8 : std::string::npos;
+        if (at != std::string::npos) {
+            size_t end = m.find(':', at);
+            m = "program " + std::to_string(start[k] + std::stoul(m.substr(at, end - at))) + m.substr(end);
+        }
+        sync_both();
+        return fail(rc, m);
+    };
+    int rc = begin(0);
+    if (rc) return plan_fail(rc, 0);
     for (uint32_t k = 0; k < n_chunks; ++k) {
         const uint32_t s0 = start[k], cnt = start[k + 1] - s0;
-        rsr_population sub = pop;
-        sub.n_programs = cnt;
-        sub.code_off = pop.code_off + s0;
-        sub.kind_off = pop.kind_off + s0;
-        sub.param_off = pop.param_off + s0;
-        int rc = build_plan(ctx, sub, dsp ? dsp + s0 : nullptr, ds, kernel, gradient, MODE_MSE, &plans[k]);
-        if (rc) {
-            // report the program by its index in the caller's population
-            std::string m = rsr_last_error();
-            const size_t at = m.rfind("program ", 0) == 0 ? 8 : std::string::npos;
-            if (at != std::string::npos) {
-                size_t end = m.find(':', at);
-                m = "program " + std::to_string(s0 + std::stoul(m.substr(at, end - at))) + m.substr(end);
-            }
-            sync_both();
-            return fail(rc, m);
+        wait_plan(ctx, &ctx->enc[k & 1]);
+        // an error of chunk k is reported before one that chunk k + 1 begins with
+        const int next = k + 1 < n_chunks ? begin(k + 1) : RSR_OK;
+        const std::string next_msg = next ? rsr_last_error() : "";
+        rc = end_plan(ctx, part_of(k), &plans[k], &ctx->enc[k & 1], nullptr);
+        if (rc || next) {
+            if (!next && k + 1 < n_chunks) wait_plan(ctx, &ctx->enc[(k + 1) & 1]);
+            if (!rc) fail(next, next_msg);
+            return rc ? plan_fail(rc, k) : plan_fail(next, k + 1);
         }
+        auto stop = [&](int code) {
+            if (k + 1 < n_chunks) wait_plan(ctx, &ctx->enc[(k + 1) & 1]);
+            sync_both();
+            return code;
+        };
         DevicePlan *dev = &ctx->pipe[k & 1];
         cudaStream_t st = (k & 1) ? ctx->stream2 : ctx->stream;
-        if ((rc = upload_plan(ctx, plans[k], dev, st))) { sync_both(); return rc; }
+        if ((rc = upload_plan(ctx, plans[k], dev, st))) return stop(rc);
         h2d += ctx->last_h2d;
-        if ((rc = enqueue_plan(ctx, plans[k], dev, st, nullptr))) { sync_both(); return rc; }
+        if ((rc = enqueue_plan(ctx, plans[k], dev, st, nullptr))) return stop(rc);
         if ((e = cudaMemcpyAsync(res + (size_t)s0 * stride, dev->out.p, (size_t)cnt * stride * sizeof(float),
-                                 cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
-            sync_both();
-            return cuda_fail(e, "result download");
-        }
+                                 cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+            return stop(cuda_fail(e, "result download"));
     }
     if ((e = cudaStreamSynchronize(ctx->stream2)) != cudaSuccess) return cuda_fail(e, "evaluation");
     if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cuda_fail(e, "evaluation");
@@ -1047,6 +1156,7 @@ int rsr_ctx_create(int device, const rsr_options *opts, rsr_ctx **out) {
     if (prop.major != 10) return fail(RSR_ENODEV, std::string("sm_100 device required, found ") + prop.name);
     if ((e = cudaSetDevice(device)) != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
     auto *ctx = new rsr_ctx();
+    for (EncodeScratch &s : ctx->enc) s.shared_pool = true;
     ctx->device = device;
     ctx->num_sms = prop.multiProcessorCount;
     ctx->smem_per_sm = prop.sharedMemPerMultiprocessor;

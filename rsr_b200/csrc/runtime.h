@@ -23,26 +23,28 @@
 namespace rsr {
 
 // A fixed set of host threads for data-parallel host work (program
-// encoding): run(n, f) calls f(0..n-1) across the threads and returns when
-// all calls are done.  One caller at a time (build_plan runs under the
-// context's lock).
+// encoding): begin(n, f) has f(0..n-1) called across the threads, end() takes
+// part and returns when all calls are done.  One caller and one job at a time
+// (planning runs under the context's lock, or in the slot that owns the pool).
 class TaskPool {
   public:
     explicit TaskPool(unsigned threads);
     ~TaskPool();
-    unsigned size() const { return (unsigned)threads_.size() + 1; }
-    void run(uint32_t n, const std::function<void(uint32_t)> &f);
+    void begin(uint32_t n, std::function<void(uint32_t)> f);
+    void end();
 
   private:
+    struct Job {
+        std::function<void(uint32_t)> f;
+        uint32_t n = 0;
+        std::atomic<uint32_t> next{0}, done{0};
+    };
     void work();
+    void help(Job &j);
     std::vector<std::thread> threads_;
     std::mutex mu_;
     std::condition_variable cv_, done_cv_;
-    const std::function<void(uint32_t)> *task_ = nullptr;
-    uint32_t n_ = 0;
-    std::atomic<uint32_t> next_{0};
-    size_t finished_ = 0;
-    uint64_t epoch_ = 0;
+    std::shared_ptr<Job> job_;
     bool stop_ = false;
 };
 
@@ -184,6 +186,21 @@ struct DevicePlan {
     }
 };
 
+// Encoding storage and threads of one planner: a caller that plans with its
+// own (a serving slot) needs the context's lock only for the dataset and
+// tuning tables, not for the encoding.
+struct EncodeScratch {
+    std::vector<EncodedProgram> enc;
+    std::vector<int> rc;
+    std::vector<std::string> msg;
+    std::vector<int> path;            // launch of each program (runtime.cu)
+    std::vector<uint8_t> adj_omit;
+    std::vector<uint32_t> prog_ds;    // index into the plan's datasets
+    bool running = false;             // encoding threads at work for this planner
+    bool shared_pool = false;         // encodes on the context's threads
+    std::unique_ptr<TaskPool> pool;
+    unsigned threads = 16;  // capped by the host's hardware threads
+};
 }  // namespace rsr
 
 struct rsr_ctx {
@@ -203,13 +220,12 @@ struct rsr_ctx {
     rsr::DevicePlan scratch;   // for one-shot calls
     rsr::DevicePlan pipe[2];   // one-shot calls split into chunks, alternating
     rsr::HostBuf results;      // pinned results of a chunked one-shot call
-    std::unique_ptr<rsr::TaskPool> encoders;  // host threads for program encoding
     // Kept between calls so that encoding and planning a population of a
     // size seen before allocates nothing new: one encoding per program of
-    // the largest population so far, and the plans of one-shot calls.
-    std::vector<rsr::EncodedProgram> enc_cache;
-    std::vector<int> enc_rc;
-    std::vector<std::string> enc_msg;
+    // the largest population (or chunks, which alternate) so far, the host
+    // threads that encode, and the plans of one-shot calls.
+    rsr::EncodeScratch enc[2];   // both on the context's encoding threads
+    std::unique_ptr<rsr::TaskPool> encoders;
     std::vector<rsr::Plan> call_plans;
     void *l2buf = nullptr;
     size_t l2bytes = 0;
@@ -232,16 +248,6 @@ struct rsr_batch {
 };
 
 namespace rsr {
-// Encoding storage and threads of one planner: a caller that plans with its
-// own (a serving slot) needs the context's lock only for the dataset and
-// tuning tables, not for the encoding.
-struct EncodeScratch {
-    std::vector<EncodedProgram> enc;
-    std::vector<int> rc;
-    std::vector<std::string> msg;
-    std::unique_ptr<TaskPool> pool;
-    unsigned threads = 16;  // capped by the host's hardware threads
-};
 // Planning and execution (runtime.cu), shared with the serving loop.
 // scratch == nullptr: the context's own encoding storage and threads (the
 // caller holds ctx->mu).  With scratch, table_mu (ctx->mu) is taken only
