@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
     io.tm = opaque(meta[1] + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(warp >> 2) * a.tmem_cols);
 
     for (;;) {
-        if (threadIdx.x == 0) meta[0] = atomicAdd(a.item_counter, 1u);
+        if (threadIdx.x == 0) meta[0] = next_item(a.item_counter, a.n_items);
         __syncthreads();
         const uint32_t item_id = meta[0];
         if (item_id >= a.n_items) break;
@@ -754,7 +754,20 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
             double s = 0.0;
             if (k <= np)
                 for (int w = 0; w < nw; ++w) s += red[((size_t)part * nw + w) * (1 + kAdjParams) + k];
-            a.partials[(size_t)(pd.part_off + it.chunk + part) * (1 + kAdjParams) + k] = s;
+            if (!a.mse_out) {
+                a.partials[(size_t)(pd.part_off + it.chunk + part) * (1 + kAdjParams) + k] = s;
+                continue;
+            }
+            // the program's only part: its results (evaluator.rs:211-223)
+            double e = 0.0;
+            for (int w = 0; w < nw; ++w) e += red[(size_t)w * (1 + kAdjParams)];
+            float m;
+            const bool ok = mse_of_sum(e, ds.num_samples, &m);
+            if (k == 0)
+                a.mse_out[it.prog_begin] = m;
+            else
+                a.grad_out[(size_t)it.prog_begin * kAdjParams + k - 1] =
+                    ok && k <= np ? (float)(s / (double)ds.num_samples) : 0.0f;
         }
         __syncthreads();
     }

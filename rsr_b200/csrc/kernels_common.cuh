@@ -24,7 +24,9 @@ struct LaunchArgs {
     double *partials;         // per (program, chunk) sums; gradient: (1+32) per slot
     float *points_out;        // MODE_POINTS: predictions
     uint64_t points_stride;   // MODE_POINTS: floats between consecutive programs
-    uint32_t *item_counter;   // persistent kernels: next work item
+    uint32_t *item_counter;   // persistent kernels: next work item; 0 before and after a launch
+    float *mse_out;           // register kernels, when every program has one part: the epilogue's
+    float *grad_out;          // results, written by the item's block (no finalize launch); else null
     uint32_t *status;         // sticky error flags (bit 0: bad micro-op)
     const uint8_t *active;    // optional per-program mask (launch order): 0 = skip
     const uint32_t *run_if;   // optional: the launch does nothing when *run_if == 0 (device-side
@@ -76,6 +78,25 @@ struct Kahan {
     }
     __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
+
+// The epilogue of compute_mse (evaluator.rs:166-173): a sum that the
+// reference's f32 accumulator would have overflowed, or a quotient that is not
+// finite, gives f32::MAX (returns false).
+__device__ __forceinline__ bool mse_of_sum(double s, uint64_t num_samples, float *mse) {
+    const float m = (float)(s / (double)num_samples);
+    const bool ok = s <= (double)3.402823466e38f && fabsf(m) <= 3.402823466e38f;
+    *mse = ok ? m : 3.402823466e38f;
+    return ok;
+}
+
+// The next work item of a persistent launch.  Every block ends on one number
+// past the last item; the block that draws the last of those sets the counter
+// back to 0 for the plan's next launch.
+__device__ __forceinline__ uint32_t next_item(uint32_t *counter, uint32_t n_items) {
+    const uint32_t id = atomicAdd(counter, 1u);
+    if (id == n_items + gridDim.x - 1u) *counter = 0u;
+    return id;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

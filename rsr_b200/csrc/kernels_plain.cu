@@ -186,9 +186,8 @@ __global__ void finalize_mse_kernel(const ProgDesc *progs, const DatasetDesc *da
     const ProgDesc pd = progs[p];
     double s = 0.0;
     for (uint32_t c = 0; c < pd.n_parts; ++c) s += partials[pd.part_off + c];
-    const double n = (double)datasets[pd.dataset].num_samples;
-    float m = (float)(s / n);
-    if (!(s <= (double)FLT_MAX) || !isfinite(m)) m = FLT_MAX;
+    float m;
+    mse_of_sum(s, datasets[pd.dataset].num_samples, &m);
     mse_out[p] = m;
 }
 

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
     for (int t = 0; t < N_STACKS; ++t) io.stk[t] = opaque(smem_addr(wbase + a.stack_off[t] + lane_point<P>(lane, 0)));
 
     for (;;) {
-        if (threadIdx.x == 0) meta[24] = atomicAdd(a.item_counter, 1u);
+        if (threadIdx.x == 0) meta[24] = next_item(a.item_counter, a.n_items);
         __syncthreads();
         const uint32_t item_id = meta[24];
         if (item_id >= a.n_items) break;
@@ -293,7 +293,11 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
             if (threadIdx.x < G) {
                 double s = 0.0;
                 for (int w = 0; w < nw; ++w) s += red[w * kMaxProgsPerWarp + threadIdx.x];
-                a.partials[a.progs[it.prog_begin + threadIdx.x].part_off + it.chunk] = s;
+                const uint32_t p = it.prog_begin + threadIdx.x;
+                if (a.mse_out)
+                    mse_of_sum(s, ds.num_samples, a.mse_out + p);
+                else
+                    a.partials[a.progs[p].part_off + it.chunk] = s;
             }
         }
         __syncthreads();

@@ -418,9 +418,7 @@ int fit_population(rsr_ctx *ctx, const rsr_population *pop, const uint64_t *dsp,
     if (exec) {
         // launches of the replays: per iteration the direction, line-search,
         // gradient-point and update kernels plus the two plans' launches
-        uint64_t per_plan_g = 1, per_plan_m = 1;
-        for (const Group &g : gev.plan.groups) per_plan_g += g.n_items ? 1 : 0;
-        for (const Group &g : mev.plan.groups) per_plan_m += g.n_items ? 1 : 0;
+        const uint64_t per_plan_g = gev.plan.launches(), per_plan_m = mev.plan.launches();
         ctx->launches += replays * (3 + kRounds + kRounds * per_plan_m + per_plan_g);
         cudaGraphExecDestroy(exec);
     }
@@ -457,6 +455,15 @@ extern "C" int rsr_fit_lbfgs(rsr_ctx *ctx, const rsr_population *pop, rsr_datase
     if (!ctx || !pop || !params_out || !mse_out) return fail(RSR_EINVAL, "null argument");
     std::lock_guard<std::mutex> lk(ctx->mu);
     cudaSetDevice(ctx->device);
-    return fit_population(ctx, pop, dsp, ds, max_iterations, ctx->stream, nullptr, nullptr, nullptr, params_out,
-                          mse_out, stats);
+    // The buffers stay for the context's next fit, up to a size: allocating
+    // and freeing them (pinned memory above all) took 1 to 5 ms a call.
+    constexpr size_t kKeepBytes = (size_t)256 << 20;
+    if (!ctx->fit) ctx->fit = std::make_unique<FitWorkspace>();
+    const int rc = fit_population(ctx, pop, dsp, ds, max_iterations, ctx->stream, nullptr, nullptr, ctx->fit.get(),
+                                  params_out, mse_out, stats);
+    if (ctx->fit->bytes() > kKeepBytes) {
+        cudaStreamSynchronize(ctx->stream);
+        ctx->fit.reset();
+    }
+    return rc;
 }

@@ -175,6 +175,8 @@ static constexpr uint64_t kStrideAlign = 1024;   // dataset column padding
 static constexpr int kGradSlotDoubles = 33;      // sse + 32 gradient sums
 
 static uint64_t round_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
+// Work items an SM of a plan whose profiles run as one launch each.
+static constexpr uint64_t kMergeItemsPerSm = 2;
 static int log2_bucket(uint64_t n) {
     int b = 0;
     while ((1ull << (b + 1)) <= n) ++b;
@@ -311,6 +313,70 @@ static void sort_by_key(std::vector<std::pair<uint64_t, uint32_t>> *v, std::vect
     }
 }
 
+// Splitting a profile's programs into launches by spill depth and by handler
+// set pays when each launch fills the device.  A small plan's launches would
+// only add their own latency, a fork and a join: up to kMergeItemsPerSm items an
+// SM the spill depths share a launch, and up to one item on every other SM the
+// handler sets do too.  1024 scalar programs x 400 points, resident: 74 us as
+// three launches with a counter reset and a finalize launch, 55 us as one
+// launch without them.  Not where the deepest program's stacks would cost the others points
+// per lane (end_plan halves P until a block fits) or the datasets' sizes ask
+// for different ones, so that no program's result depends on it.
+static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *S, uint32_t n, std::mutex *table_mu) {
+    auto items_of = [&](uint32_t i) { return (plan.datasets[S->prog_ds[i]].n_eval + kChunkPoints - 1) / kChunkPoints; };
+    uint64_t total = 0;
+    for (uint32_t i = 0; i < n; ++i) total += items_of(i);
+    if (total > 8ull * kMergeItemsPerSm * (uint64_t)ctx->num_sms) return;  // even at 8 programs an item
+    for (int prof = 0; prof < N_PROFILES; ++prof)
+        for (int set = -1; set < 4; ++set) {  // all handler sets together, then each by itself
+            unsigned omit = ~0u;
+            int cls = 0, first = -1;
+            bool split = false;
+            uint32_t cw = 0, cf = 0, depth[N_STACKS] = {0, 0, 0, 0, 0};
+            uint64_t items = 0, lo = ~0ull, hi = 0;
+            auto member = [&](uint32_t i) {
+                const int p = S->path[i];
+                return p >= 0 && p % kRegPathStride == prof && (set < 0 || p / kRegPathStride / 3 == set);
+            };
+            for (uint32_t i = 0; i < n; ++i) {
+                if (!member(i)) continue;
+                const int p = S->path[i];
+                const EncodedProgram &E = S->enc[i];
+                const uint64_t n_eval = plan.datasets[S->prog_ds[i]].n_eval;
+                if (first < 0) first = p;
+                split |= p != first;
+                omit &= (unsigned)(p / kRegPathStride / 3);
+                cls = std::max(cls, p / kRegPathStride % 3);
+                cw = std::max(cw, (uint32_t)E.reg_code.size() + 1);
+                cf = std::max(cf, (uint32_t)E.consts.size() + E.n_hoist);
+                for (int t = 0; t < N_STACKS; ++t) depth[t] = std::max(depth[t], (uint32_t)E.depth_fast[t]);
+                lo = std::min(lo, n_eval);
+                hi = std::max(hi, n_eval);
+                items += items_of(i);
+            }
+            if (!split) continue;
+            TuneChoice c;
+            {
+                std::unique_lock<std::mutex> lock;
+                if (table_mu) lock = std::unique_lock<std::mutex>(*table_mu);
+                c = choice_for(ctx, prof, hi);
+                bool same = true;
+                for (int b = log2_bucket(std::max<uint64_t>(lo, 1)); b <= log2_bucket(std::max<uint64_t>(hi, 1)); ++b) {
+                    const TuneChoice d = choice_for(ctx, prof, std::min(std::max(1ull << b, (unsigned long long)lo), (unsigned long long)hi));
+                    same = same && d.P == c.P && d.G == c.G;
+                }
+                if (!same) continue;
+            }
+            const uint64_t most = set < 0 ? (uint64_t)ctx->num_sms / 2 : kMergeItemsPerSm * (uint64_t)ctx->num_sms;
+            if (items > (uint64_t)c.G * most) continue;
+            if (reg_smem_bytes(cw * (uint32_t)c.G, cf * (uint32_t)c.G, depth, c.P, c.G) > kRegSmemBudget) continue;
+            const int merged = prof + kRegPathStride * (cls + 3 * (int)omit);
+            for (uint32_t i = 0; i < n; ++i)
+                if (member(i)) S->path[i] = merged;
+            if (set < 0) break;
+        }
+}
+
 // Planning in two halves.  begin_plan looks the datasets up and starts
 // encoding the programs, each only in the form its kernel needs, on the
 // encoding threads; end_plan waits for them and lays the launch out.  Between
@@ -427,6 +493,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
     for (uint32_t i = 0; i < n; ++i)
         if (S->rc[i] != RSR_OK) return fail(S->rc[i], "program " + std::to_string(i) + ": " + S->msg[i]);
     std::unique_lock<std::mutex> table_lock;
+    if (!gradient) merge_small_launches(ctx, P, S, n, table_mu);
     // group programs by (path, dataset), each group sorted by descending code length
     // (one 64-bit key per program: path, dataset, then longer code first and
     // the caller's order among equals, as a stable sort by those would give)
@@ -662,6 +729,9 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
         P.groups.push_back(g);
         li = end;
     }
+    P.one_part = P.mode == MODE_MSE;
+    for (const ProgDesc &d : P.progs) P.one_part = P.one_part && d.n_parts == 1;
+    for (const Group &g : P.groups) P.one_part = P.one_part && (g.kind == 1 || g.kind == 3);
     // Launches run side by side (enqueue_plan): the one whose longest item
     // takes longest goes first, so that it does not become the plan's tail.
     std::stable_sort(P.groups.begin(), P.groups.end(),
@@ -695,7 +765,8 @@ int upload_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t st
     const size_t o_items = o_ds + al(plan.datasets.size() * sizeof(DatasetDesc));
     const size_t o_code = o_items + al(plan.items.size() * sizeof(WorkItem));
     const size_t o_consts = o_code + al((plan.code.size() + 1) * sizeof(uint32_t));
-    const size_t total = o_consts + al((plan.consts.size() + 1) * sizeof(float));
+    const size_t o_count = o_consts + al((plan.consts.size() + 1) * sizeof(float));
+    const size_t total = o_count + al(std::max<size_t>(plan.groups.size(), 1) * sizeof(uint32_t));
     cudaError_t e;
     if ((e = dev->pool.reserve(total)) != cudaSuccess) return cuda_fail(e, "plan pool");
     if ((e = dev->partials.reserve(std::max<size_t>(plan.n_partials, 1) * sizeof(double))) != cudaSuccess)
@@ -704,8 +775,6 @@ int upload_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t st
     if (plan.raw_sums) out_floats *= 2;  // doubles
     if ((e = dev->out.reserve(std::max<size_t>(out_floats, 1) * sizeof(float))) != cudaSuccess)
         return cuda_fail(e, "outputs");
-    if ((e = dev->counters.reserve(std::max<size_t>(plan.groups.size(), 1) * sizeof(uint32_t) + 64)) != cudaSuccess)
-        return cuda_fail(e, "counters");
     // the staging buffer may still feed this plan's previous copy
     if (dev->staged) {
         if ((e = cudaEventSynchronize(dev->staged)) != cudaSuccess) return cuda_fail(e, "staging wait");
@@ -729,6 +798,7 @@ int upload_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t st
     memcpy(h + o_items, plan.items.data(), plan.items.size() * sizeof(WorkItem));
     memcpy(h + o_code, plan.code.data(), plan.code.size() * sizeof(uint32_t));
     memcpy(h + o_consts, plan.consts.data(), plan.consts.size() * sizeof(float));
+    memset(h + o_count, 0, total - o_count);  // the kernels leave their counters at 0
     if ((e = cudaMemcpyAsync(dev->pool.p, h, total, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return cuda_fail(e, "plan upload");
     if ((e = cudaEventRecord(dev->staged, st)) != cudaSuccess) return cuda_fail(e, "staging event");
@@ -741,6 +811,7 @@ int upload_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t st
     a.items = (const WorkItem *)(d + o_items);
     a.code = (const uint32_t *)(d + o_code);
     a.consts = (const float *)(d + o_consts);
+    a.item_counter = (uint32_t *)(d + o_count);
     a.partials = (double *)dev->partials.p;
     a.mode = (uint32_t)plan.mode;
     a.points_stride = plan.points_stride;
@@ -813,9 +884,6 @@ int enqueue_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t s
         return RSR_OK;
     }
     cudaError_t e;
-    uint32_t *counters = (uint32_t *)dev->counters.p;
-    if ((e = cudaMemsetAsync(counters, 0, plan.groups.size() * sizeof(uint32_t), st)) != cudaSuccess)
-        return cuda_fail(e, "counter reset");
     // Launch j > 0 goes to side stream (j - 1) % 2 unless per-launch timing is
     // asked for (events around each launch then time it alone).  Launches
     // share nothing but the partials, which each item writes at its own index.
@@ -838,7 +906,11 @@ int enqueue_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t s
         LaunchArgs a = dev->base;
         a.items = dev->base.items + g.item_begin;
         a.n_items = g.n_items;
-        a.item_counter = counters + gi;
+        a.item_counter = dev->base.item_counter + gi;
+        if (plan.results_in_kernel()) {
+            a.mse_out = dev->mse;
+            a.grad_out = dev->grad;
+        }
         a.smem_code_words = g.code_words;
         a.smem_const_floats = g.const_floats;
         a.smem_slots = g.slots;
@@ -911,7 +983,7 @@ int enqueue_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t s
                                  (double *)dev->out.p, st);
         if (e != cudaSuccess) return cuda_fail(e, "finalize launch");
         ctx->launches++;
-    } else if (plan.mode == MODE_MSE) {
+    } else if (plan.mode == MODE_MSE && !plan.results_in_kernel()) {
         if (plan.gradient)
             e = launch_finalize_grad(dev->base.progs, dev->base.datasets, dev->base.partials, n, dev->mse, dev->grad, st);
         else
@@ -939,15 +1011,18 @@ static int fetch_results(rsr_ctx *ctx, const Plan &plan, DevicePlan &dev, cudaSt
         for (size_t li = 0; li < n; ++li) memcpy(points_out + (size_t)plan.orig[li] * per, tmp.data() + li * per, per * sizeof(float));
         return RSR_OK;
     }
+    // through pinned memory: a copy to pageable memory goes through the
+    // driver's own staging, one more copy and synchronisation
     const size_t nf = n * (plan.gradient ? 33 : 1);
-    std::vector<float> tmp(nf);
-    if ((e = cudaMemcpyAsync(tmp.data(), dev.out.p, nf * sizeof(float), cudaMemcpyDeviceToHost, st)))
+    if ((e = ctx->results.reserve(nf * sizeof(float))) != cudaSuccess) return cuda_fail(e, "cudaHostAlloc");
+    const float *tmp = (const float *)ctx->results.p;
+    if ((e = cudaMemcpyAsync(ctx->results.p, dev.out.p, nf * sizeof(float), cudaMemcpyDeviceToHost, st)))
         return cuda_fail(e, "result download");
     if ((e = cudaStreamSynchronize(st))) return cuda_fail(e, "evaluation");
     ctx->last_d2h = nf * sizeof(float);
     for (size_t li = 0; li < n; ++li) {
         if (mse_out) mse_out[plan.orig[li]] = tmp[li];
-        if (grad_out && plan.gradient) memcpy(grad_out + (size_t)plan.orig[li] * 32, tmp.data() + n + li * 32, 32 * sizeof(float));
+        if (grad_out && plan.gradient) memcpy(grad_out + (size_t)plan.orig[li] * 32, tmp + n + li * 32, 32 * sizeof(float));
     }
     (void)ctx;
     return RSR_OK;
@@ -1191,12 +1266,12 @@ int rsr_ctx_destroy(rsr_ctx *ctx) {
     ctx->scratch.pool.release();
     ctx->scratch.partials.release();
     ctx->scratch.out.release();
-    ctx->scratch.counters.release();
     ctx->scratch.staging.release();
     for (DevicePlan &d : ctx->pipe) {
-        d.pool.release(); d.partials.release(); d.out.release(); d.counters.release(); d.staging.release();
+        d.pool.release(); d.partials.release(); d.out.release(); d.staging.release();
     }
     ctx->results.release();
+    ctx->fit.reset();
     if (ctx->l2buf) cudaFree(ctx->l2buf);
     for (auto &ev : ctx->ev) if (ev) cudaEventDestroy(ev);
     cudaStreamDestroy(ctx->stream);
@@ -1427,9 +1502,7 @@ int rsr_batch_run(rsr_ctx *ctx, rsr_batch *b) {
         }
         cudaEventRecord(b->ev[0], ctx->stream);
         if ((e = cudaGraphLaunch(b->graph, ctx->stream)) != cudaSuccess) return cuda_fail(e, "graph launch");
-        uint64_t nl = 0;
-        for (auto &g : b->plan.groups) nl += g.n_items ? 1 : 0;
-        ctx->launches += nl + (b->plan.progs.empty() ? 0 : 1);
+        ctx->launches += b->plan.launches();
         cudaEventRecord(b->ev[2], ctx->stream);
         return RSR_OK;
     }
@@ -1612,7 +1685,7 @@ int rsr_autotune(rsr_ctx *ctx, const rsr_population *pop, rsr_dataset ds, const 
         }
     ctx->force = TuneChoice{};
     for (auto &e : ev) cudaEventDestroy(e);
-    dev.pool.release(); dev.partials.release(); dev.out.release(); dev.counters.release();
+    dev.pool.release(); dev.partials.release(); dev.out.release();
     if (rc) return rc;
     rep += "], \"chosen\": [";
     first = true;

@@ -136,11 +136,22 @@ struct Plan {
     uint32_t n_partials = 0;                // doubles (gradient: 33 per slot)
     bool gradient = false;
     bool raw_sums = false;                  // MODE_MSE: unscaled f64 sums instead of the epilogue
+    bool one_part = false;                  // MODE_MSE: every program has one part and runs on a register kernel
     int mode = MODE_MSE;
     uint64_t points_stride = 0;
     uint64_t flops = 0;                     // algorithmic lane-ops of one run
     uint64_t program_points = 0;
     uint32_t n_plain = 0, n_reg = 0;
+
+    // The kernels write the results themselves; otherwise a finalize launch
+    // follows the groups'.
+    bool results_in_kernel() const { return one_part && !raw_sums; }
+    // Kernel launches of one run.
+    uint64_t launches() const {
+        uint64_t n = progs.empty() || mode != MODE_MSE || results_in_kernel() ? 0 : 1;
+        for (const Group &g : groups) n += g.n_items ? 1 : 0;
+        return n;
+    }
 
     // Empty, with the vectors' capacity kept for the next build.
     void reset() {
@@ -159,11 +170,9 @@ struct Plan {
 
 // Device copy of a plan plus the buffers one run writes.
 struct DevicePlan {
-    DevBuf pool;        // progs | datasets | items | code | consts
+    DevBuf pool;        // progs | datasets | items | code | consts | item counters
     DevBuf partials;
     DevBuf out;         // mse (n floats) [+ grad (n*32 floats)]
-    DevBuf counters;    // one item counter per group
-    DevBuf status;
     HostBuf staging;    // pinned image of the pool, uploaded with one copy
     cudaEvent_t staged = nullptr;  // recorded after the staging buffer's copy
     // Every launch of a plan but the first goes to one of two side streams,
@@ -183,6 +192,19 @@ struct DevicePlan {
             if (join[i]) cudaEventDestroy(join[i]);
             if (side[i]) cudaStreamDestroy(side[i]);
         }
+    }
+};
+
+// Buffers of a batched L-BFGS fit.
+struct FitWorkspace {
+    DevicePlan grad, mse;
+    DevBuf grad_active, mse_active;
+    DevBuf lbfgs_state;   // device-resident L-BFGS state of every program (lbfgs.cu)
+    HostBuf lbfgs_counts; // pinned copy of the per-iteration counters
+    size_t bytes() const {
+        size_t n = grad_active.cap + mse_active.cap + lbfgs_state.cap;
+        for (const DevicePlan *d : {&grad, &mse}) n += d->pool.cap + d->partials.cap + d->out.cap + d->staging.cap;
+        return n;
     }
 };
 
@@ -227,6 +249,7 @@ struct rsr_ctx {
     rsr::EncodeScratch enc[2];   // both on the context's encoding threads
     std::unique_ptr<rsr::TaskPool> encoders;
     std::vector<rsr::Plan> call_plans;
+    std::unique_ptr<rsr::FitWorkspace> fit;  // buffers of rsr_fit_lbfgs (lbfgs.cu)
     void *l2buf = nullptr;
     size_t l2bytes = 0;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -266,12 +289,6 @@ rsr_dataset register_dataset(rsr_ctx *ctx, std::unique_ptr<DatasetRec> rec);
 // plans are built (they read the context's dataset and tuning tables);
 // cancel, when set, stops the fit between iterations with RSR_ECANCELED.
 // ws, when given, supplies (and keeps) the device buffers of the fit.
-struct FitWorkspace {
-    DevicePlan grad, mse;
-    DevBuf grad_active, mse_active;
-    DevBuf lbfgs_state;   // device-resident L-BFGS state of every program (lbfgs.cu)
-    HostBuf lbfgs_counts; // pinned copy of the per-iteration counters
-};
 int fit_population(rsr_ctx *ctx, const rsr_population *pop, const uint64_t *dsp, uint64_t ds,
                    uint32_t max_iterations, cudaStream_t stream, std::mutex *plan_mu,
                    const std::atomic<bool> *cancel, FitWorkspace *ws, float *params_out, float *mse_out,

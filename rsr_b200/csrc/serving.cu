@@ -90,10 +90,10 @@ struct Slot {
                fit.mse.partials.cap + fit.mse.out.cap;
     }
     void trim() {
-        dev.pool.release(); dev.partials.release(); dev.out.release(); dev.counters.release();
-        dev2.pool.release(); dev2.partials.release(); dev2.out.release(); dev2.counters.release();
+        dev.pool.release(); dev.partials.release(); dev.out.release();
+        dev2.pool.release(); dev2.partials.release(); dev2.out.release();
         for (DevicePlan *d : {&fit.grad, &fit.mse}) {
-            d->pool.release(); d->partials.release(); d->out.release(); d->counters.release();
+            d->pool.release(); d->partials.release(); d->out.release();
         }
         fit.grad_active.release();
         fit.mse_active.release();
