@@ -354,30 +354,45 @@ __device__ __forceinline__ void rev_op(Acc<PROF, P> &g, const RevIO<P> &io, uint
                 constexpr int tm = W == 2 ? SM2 : SM3;
                 constexpr int MW = W * W;
                 if constexpr (((kProfileTypes[PROF] >> tm) & 1u) != 0u || k != km) {
-                    Vf<P> v[W], m[MW], gm[MW];
-                    load_tape<P, W>(v, io, ta);
-                    if constexpr (k == km) load_tape<P, MW>(m, io, tb);
-                    else fetch<P, MW, k - km - 1>(m, io, tm, arg);
-#pragma unroll
-                    for (int c = 0; c < W; ++c)
-#pragma unroll
-                        for (int r = 0; r < W; ++r) gm[W * c + r] = G[r] * v[c];
-                    if constexpr (k == km) {
-                        if constexpr (((kProfileTypes[PROF] >> tm) & 1u) != 0u) {
-                            Vf<P> *GM = acc_of<PROF, P, tm>(g);
-#pragma unroll
-                            for (int i = 0; i < MW; ++i) GM[i] = GM[i] + gm[i];
-                        }
-                    } else {
-                        send<P, MW, k - km - 1>(io, tm, arg, gm);
-                    }
-                    Vf<P> nv[W];
+                    // a column of the matrix at a time, its adjoints sent as
+                    // they are formed: the whole matrix and its adjoint are
+                    // 144 registers at 8 points per lane
+                    constexpr int src = k - km - 1;
+                    Vf<P> v[W], nv[W];
+                    if constexpr (src != SRC_X) load_tape<P, W>(v, io, ta);
 #pragma unroll
                     for (int c = 0; c < W; ++c) {
+                        Vf<P> m[W];
+                        if constexpr (k == km) {
+                            load_tape<P, W>(m, io, tb + (uint32_t)(c * W));
+                        } else {
+#pragma unroll
+                            for (int r = 0; r < W; ++r) {
+                                if constexpr (src == SRC_X) m[r] = io.X(arg + W * c + r);
+                                else if constexpr (src == SRC_C) m[r] = io.C(arg + W * c + r);
+                                else m[r] = io.template S<MW>(tm, arg, W * c + r);
+                            }
+                        }
                         Vf<P> s = splat<P>(0.0f);
 #pragma unroll
-                        for (int r = 0; r < W; ++r) s = s + m[W * c + r] * G[r];
+                        for (int r = 0; r < W; ++r) s = s + m[r] * G[r];
                         nv[c] = s;
+                        if constexpr (src != SRC_X) {
+#pragma unroll
+                            for (int r = 0; r < W; ++r) {
+                                const Vf<P> gm = G[r] * v[c];
+                                if constexpr (k == km) {
+                                    if constexpr (((kProfileTypes[PROF] >> tm) & 1u) != 0u) {
+                                        Vf<P> *GM = acc_of<PROF, P, tm>(g);
+                                        GM[W * c + r] = GM[W * c + r] + gm;
+                                    }
+                                } else if constexpr (src == SRC_C) {
+                                    io.grad_add(arg + W * c + r, gm);
+                                } else {
+                                    io.template put_g<MW>(tm, arg, W * c + r, gm);
+                                }
+                            }
+                        }
                     }
 #pragma unroll
                     for (int c = 0; c < W; ++c) G[c] = nv[c];
@@ -517,6 +532,9 @@ __device__ __forceinline__ void fwd_op(Acc<PROF, P> &a, const RevIO<P> &io, uint
 #define RSR_ADJ_F(M) RSR_X27(M, K_F)
 #define RSR_ADJ_F_NU(M) RSR_X9(M, K_F) RSR_X9(M, K_F + 9) M(K_F + 18) M(K_F + 19) M(K_F + 20)
 #define RSR_ADJ_V3(M) RSR_X34(M, K_V3)
+// F+V3 has no Mat3 accumulator to multiply from or to spill: no mat-vec with
+// either (64 + 29, 64 + 32)
+#define RSR_ADJ_V3_F(M) RSR_X27(M, K_V3) M(K_V3 + 27) M(K_V3 + 28) M(K_V3 + 30) M(K_V3 + 31) M(K_V3 + 33)
 #define RSR_ADJ_V3_NM(M) RSR_X27(M, K_V3) M(K_V3 + 27) M(K_V3 + 28) M(K_V3 + 29) M(K_V3 + 33)
 static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec kinds at 29..32");
 #define RSR_SWITCH(M, EXTRA)                                                                          \
@@ -527,11 +545,11 @@ static_assert(kv_mulm(5, 3) == 29 && kv_make(5, 3) == 33, "Vec3 block: mat-vec k
     } else if constexpr (PROF == P_FV3 && (OMIT & 3) == 3) {                                          \
         switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3_NM(M) case K_STOP: return; default: __builtin_unreachable(); }                      \
     } else if constexpr (PROF == P_FV3 && (OMIT & 1)) {                                               \
-        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3(M) case K_STOP: return; default: __builtin_unreachable(); }                         \
+        switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_ADJ_V3_F(M) case K_STOP: return; default: __builtin_unreachable(); }                         \
     } else if constexpr (PROF == P_FV3 && (OMIT & 2)) {                                               \
         switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3_NM(M) case K_STOP: return; default: __builtin_unreachable(); }                         \
     } else if constexpr (PROF == P_FV3) {                                                             \
-        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3(M) case K_STOP: return; default: __builtin_unreachable(); }                            \
+        switch (kind) { EXTRA RSR_ADJ_F(M) RSR_ADJ_V3_F(M) case K_STOP: return; default: __builtin_unreachable(); }                            \
     } else if constexpr (PROF == P_FV2M2 && (OMIT & 1)) {                                             \
         switch (kind) { EXTRA RSR_ADJ_F_NU(M) RSR_X27(M, K_V2) RSR_X27(M, K_M2) case K_STOP: return; default: __builtin_unreachable(); }     \
     } else if constexpr (PROF == P_FV2M2) {                                                           \
@@ -585,6 +603,7 @@ __device__ __forceinline__ void run_reverse(Acc<PROF, P> &g, const RevIO<P> &io,
 #undef RSR_ADJ_F_NU
 #undef RSR_ADJ_V3
 #undef RSR_ADJ_V3_NM
+#undef RSR_ADJ_V3_F
 #undef RSR_X34
 #undef RSR_X27
 #undef RSR_X9

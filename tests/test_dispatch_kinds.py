@@ -102,8 +102,7 @@ def test_every_emitted_kind_is_in_its_profiles_table(form):
             n_fwd, n_rev = int(code[0]), int(code[1])
             assert len(code) == 2 + 2 * (n_fwd + n_rev)   # where the kernel puts its stop entries
             kinds = {int(w) & 255 for w in code[2::2]}
-            # the adjoint's tables hold every kind of a profile's types
-            table = TABLE[prof] | TAPE[prof] | ({64 + 29, 64 + 32} if prof == 1 else set())
+            table = TABLE[prof] | TAPE[prof]
         assert kinds <= table, (prof, sorted(kinds - table))
         # leaving out a handler set whose kinds do not occur keeps every kind that does
         for gone in OMITTABLE[prof]:
