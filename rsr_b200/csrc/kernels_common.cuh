@@ -203,6 +203,14 @@ __device__ __forceinline__ double lds_f64(uint32_t a) {
 __device__ __forceinline__ void sts_f64(uint32_t a, double v) {
     asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
+__device__ __forceinline__ float2 lds_f32x2(uint32_t a) {
+    float2 r;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ void sts_f32x2(uint32_t a, float x, float y) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x), "f"(y) : "memory");
+}
 __device__ __forceinline__ float lds_f32(uint32_t a) { return __uint_as_float(lds_u32(a)); }
 
 // Shared-memory image of a lane's P values in a block of 32*P floats; a is

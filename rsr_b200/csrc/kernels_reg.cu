@@ -114,7 +114,20 @@ __host__ __device__ __forceinline__ uint32_t align4r(uint32_t v) { return (v + 3
 
 constexpr uint32_t kMaxProgsPerWarp = 8;
 static_assert(kMaxProgsPerWarp <= kRegThreads / 32, "a warp for each program's prologue");
-constexpr uint32_t kNone = 0xFFFFFFFFu;
+constexpr uint32_t kPrologue = 0xFFFFFFFFu;  // the tile that stands for an item's prologues
+constexpr uint32_t kEnd = 0xFFFFFFFFu;       // no program at this address
+
+// What a block keeps of its work item in shared memory (words).
+enum RegMeta : uint32_t {
+    M_PROGS = 0,       // [g][2] shared-memory addresses of each program's code and constants, kEnd behind the last
+    M_PROLOGUES = 18,  // [g] address of its prologue, kEnd if it has none
+    M_Y_OFF = 26,      // targets' byte distance from the features
+    M_N_EVAL = 28,     // points to count
+    M_ITEM = 30, M_FULL_TILES, M_TILE_BEGIN, M_TILE_END, M_PROG_BEGIN, M_HOISTED,
+    kMetaWords = 36
+};
+static_assert(M_PROLOGUES == M_PROGS + 2 * (kMaxProgsPerWarp + 1) && M_Y_OFF == M_PROLOGUES + kMaxProgsPerWarp &&
+              M_HOISTED + 1 == kMetaWords && kMetaWords % 4 == 0, "RegMeta layout");
 
 // Block-cooperative item loop.  All warps of a block run the same programs
 // (one work item) on different tiles of the item's chunk, so the SM's
@@ -149,22 +162,20 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
     const int nw = blockDim.x >> 5;
     uint32_t *scode = reinterpret_cast<uint32_t *>(smem);
     float *sconst = smem + align4r(a.smem_code_words);
-    // [g][3] main program, constants and prologue (kNone: none) of each
-    // program, [24] item, [25] its programs, [26..27] targets' byte distance from the features, [28..29]
-    // points to count, [30] last tile, [31] first program
-    uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + align4r(a.smem_const_floats));
-    double *red = reinterpret_cast<double *>(meta + 32);                                  // [warp][g]
+    uint32_t *meta = reinterpret_cast<uint32_t *>(sconst + align4r(a.smem_const_floats));  // RegMeta
+    double *red = reinterpret_cast<double *>(meta + kMetaWords);  // [warp][g]
     float *wbase = smem + a.block_hdr_floats + (size_t)warp * a.region_floats;
-    float *sacc = wbase + a.acc_off;  // [g][2][32] Kahan state of this warp
+    // Kahan state of this warp: (sum, compensation) of each lane, 256 bytes a program
+    const uint32_t kahan = smem_addr(wbase + a.acc_off) + 8u * lane;
 
     AccIO<P> io;
 #pragma unroll
     for (int t = 0; t < N_STACKS; ++t) io.stk[t] = opaque(smem_addr(wbase + a.stack_off[t] + lane_point<P>(lane, 0)));
 
     for (;;) {
-        if (threadIdx.x == 0) meta[24] = next_item(a.item_counter, a.n_items);
+        if (threadIdx.x == 0) meta[M_ITEM] = next_item(a.item_counter, a.n_items);
         __syncthreads();
-        const uint32_t item_id = meta[24];
+        const uint32_t item_id = meta[M_ITEM];
         if (item_id >= a.n_items) break;
         const WorkItem it = a.items[item_id];
         const uint32_t G = it.n_progs;
@@ -174,40 +185,46 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
             bool any = false;
             for (uint32_t g = 0; g < G; ++g) any |= a.active[it.prog_begin + g] != 0;
             if (!any) {
-                __syncthreads();  // meta[24] is rewritten by the next item fetch
+                __syncthreads();  // M_ITEM is rewritten by the next item fetch
                 continue;
             }
         }
-        const DatasetDesc ds = a.datasets[a.progs[it.prog_begin].dataset];
-        if (threadIdx.x == 0) {
-            uint32_t coff = 0, koff = 0;
-            for (uint32_t g = 0; g < G; ++g) {
-                const ProgDesc pd = a.progs[it.prog_begin + g];
-                meta[3 * g] = coff + pd.n_slots;
-                meta[3 * g + 1] = koff;
-                meta[3 * g + 2] = pd.n_slots ? coff : kNone;
-                scode[coff + pd.uop_len] = K_STOP;
-                coff += pd.uop_len + 1;
-                koff += pd.n_consts + pd.n_tape;
+        // The item's programs lie one after another in the code and constant
+        // pools, as they do here (every program ended by its K_STOP, followed
+        // by room for its hoisted constants), so one copy each stages them,
+        // while warp 0's lanes lay down where each begins.
+        const DatasetDesc ds = a.datasets[it.dataset];
+        const uint32_t code0 = a.progs[it.prog_begin].uop_off, const0 = a.progs[it.prog_begin].const_off;
+        const ProgDesc &last = a.progs[it.prog_begin + G - 1];
+        const uint32_t n_code = last.uop_off + last.uop_len + 1u - code0;
+        const uint32_t n_const = last.const_off + last.n_consts + last.n_tape - const0;
+        for (uint32_t i = threadIdx.x; i < n_code; i += blockDim.x) scode[i] = __ldg(a.code + code0 + i);
+        for (uint32_t i = threadIdx.x; i < n_const; i += blockDim.x) sconst[i] = __ldg(a.consts + const0 + i);
+        for (uint32_t g = 0; g < G; ++g) sts_f32x2(kahan + 256u * g, 0.0f, 0.0f);
+        if (warp == 0) {
+            bool hoisted = false;
+            if (lane < (int)G) {
+                const ProgDesc &pd = a.progs[it.prog_begin + lane];
+                const uint32_t code = smem_addr(scode + (pd.uop_off - code0));
+                hoisted = pd.n_slots != 0u;
+                meta[M_PROGS + 2 * lane] = code + 4u * pd.n_slots;
+                meta[M_PROGS + 2 * lane + 1] = smem_addr(sconst + (pd.const_off - const0));
+                meta[M_PROLOGUES + lane] = hoisted ? code : kEnd;
+            } else if (lane <= (int)kMaxProgsPerWarp) {
+                meta[M_PROGS + 2 * lane] = kEnd;
+                if (lane < (int)kMaxProgsPerWarp) meta[M_PROLOGUES + lane] = kEnd;
             }
-            *reinterpret_cast<int64_t *>(meta + 26) =
-                reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
-            *reinterpret_cast<uint64_t *>(meta + 28) = ds.n_eval;
-            meta[25] = G;
-            meta[30] = it.tile_end;
-            meta[31] = it.prog_begin;
-        }
-        __syncthreads();
-        bool hoisted = false;
-        for (uint32_t g = 0; g < G; ++g) {
-            const ProgDesc pd = a.progs[it.prog_begin + g];
-            uint32_t *code = scode + (meta[3 * g] - pd.n_slots);
-            for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) code[i] = __ldg(a.code + pd.uop_off + i);
-            for (uint32_t i = threadIdx.x; i < pd.n_consts; i += blockDim.x)
-                sconst[meta[3 * g + 1] + i] = __ldg(a.consts + pd.const_off + i);
-            hoisted |= pd.n_slots != 0u;
-            sacc[(g * 2) * 32 + lane] = 0.0f;
-            sacc[(g * 2 + 1) * 32 + lane] = 0.0f;
+            hoisted = __any_sync(0xffffffffu, hoisted);
+            if (lane == 0) {
+                *reinterpret_cast<int64_t *>(meta + M_Y_OFF) =
+                    reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
+                *reinterpret_cast<uint64_t *>(meta + M_N_EVAL) = ds.n_eval;
+                meta[M_FULL_TILES] = (uint32_t)(ds.n_eval / (32u * P));
+                meta[M_TILE_END] = it.tile_end;
+                meta[M_TILE_BEGIN] = it.tile_begin;
+                meta[M_PROG_BEGIN] = it.prog_begin;
+                meta[M_HOISTED] = hoisted;
+            }
         }
         __syncthreads();
         io.stride = opaque((uint32_t)ds.stride);
@@ -217,51 +234,44 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
         // (shared memory and L1): held in registers it would be live across
         // the interpreter, which has none to spare at three blocks an SM.
         const volatile uint32_t *vmeta = meta;
-        // The item's prologues come first, as tile kNone: warp g runs program
-        // g's (one call of the interpreter in the kernel), then the block
-        // goes on to the tiles.
-        uint32_t tile = hoisted ? kNone : it.tile_begin + warp;
+        // The item's prologues come first, as tile kPrologue: warp g runs
+        // program g's (one call of the interpreter in the kernel), then the
+        // block goes on to the tiles.
+        uint32_t tile = vmeta[M_HOISTED] ? kPrologue : it.tile_begin + warp;
         for (;;) {
-            if (tile != kNone && tile >= vmeta[30]) break;
+            if (tile != kPrologue && tile >= vmeta[M_TILE_END]) break;
             io.xl = opaque(ds.x + ((uint64_t)tile * (32u * P) + lane_point<P>(lane, 0)));
-            for (uint32_t g = tile == kNone ? (uint32_t)warp : 0u; g < vmeta[25]; ++g) {
-                const uint32_t at = vmeta[3 * g + (tile == kNone ? 2u : 0u)];
-                if (at == kNone) break;  // no prologue
-                if (a.active && !a.active[vmeta[31] + g]) {
-                    if (tile == kNone) break;
+            for (uint32_t g = tile == kPrologue ? (uint32_t)warp : 0u;; ++g) {
+                uint2 at = lds_u32x2(smem_addr(meta) + 4u * M_PROGS + 8u * g);  // code, constants
+                if (tile == kPrologue) at.x = vmeta[M_PROLOGUES + warp];
+                if (at.x == kEnd) break;  // no further program, or no prologue
+                if (a.active && !a.active[vmeta[M_PROG_BEGIN] + g]) {
+                    if (tile == kPrologue) break;
                     continue;
                 }
-                io.consts = opaque(smem_addr(sconst + vmeta[3 * g + 1]));
-                run_program<PROF, P, OMIT>(acc, io, opaque(smem_addr(scode + at)));
-                if (tile == kNone) break;
+                io.consts = opaque(at.y);
+                run_program<PROF, P, OMIT>(acc, io, opaque(at.x));
+                if (tile == kPrologue) break;
                 const Vf<P> pred = acc.F[0];
-                const int64_t y_off = *reinterpret_cast<const volatile int64_t *>(vmeta + 26);
-                const uint64_t n_eval = *reinterpret_cast<const volatile uint64_t *>(vmeta + 28);
-                const uint64_t t0 = (uint64_t)tile * (32u * P);
                 if (a.mode == MODE_POINTS) {
-                    store_lane<P>(a.points_out + (uint64_t)(vmeta[31] + g) * a.points_stride + t0, lane, pred,
-                                  t0, n_eval);
-                } else {
-                    const Vf<P> y = load_lane<P>(
-                        reinterpret_cast<const float *>(reinterpret_cast<const char *>(io.xl) + y_off));
-                    Kahan k;
-                    k.s = sacc[(g * 2) * 32 + lane];
-                    k.c = sacc[(g * 2 + 1) * 32 + lane];
-                    if (t0 + lane_point<P>(lane, P - 1) < n_eval) {
-                        // the lane's P squared errors summed pairwise, then one
-                        // compensated add per tile
-                        float sq[P];
-#pragma unroll
-                        for (int q = 0; q < P; ++q) {
-                            const float d = pred.v[q] - y.v[q];
-                            sq[q] = d * d;
-                        }
-#pragma unroll
-                        for (int h = P / 2; h > 0; h /= 2)
-#pragma unroll
-                            for (int q = 0; q < h; ++q) sq[q] = sq[q] + sq[q + h];
-                        k.add(sq[0]);
-                    } else {
+                    const uint64_t t0 = (uint64_t)tile * (32u * P);
+                    store_lane<P>(a.points_out + (uint64_t)(vmeta[M_PROG_BEGIN] + g) * a.points_stride + t0, lane,
+                                  pred, t0, *reinterpret_cast<const volatile uint64_t *>(vmeta + M_N_EVAL));
+                    continue;
+                }
+                const int64_t y_off = *reinterpret_cast<const volatile int64_t *>(vmeta + M_Y_OFF);
+                const Vf<P> y = load_lane<P>(
+                    reinterpret_cast<const float *>(reinterpret_cast<const char *>(io.xl) + y_off));
+                const float2 sc = lds_f32x2(kahan + 256u * g);
+                Kahan k;
+                k.s = sc.x;
+                k.c = sc.y;
+                bool full = tile < vmeta[M_FULL_TILES];
+                if (!full) {  // the dataset's last tile: lanes whose points all lie inside
+                    const uint64_t n_eval = *reinterpret_cast<const volatile uint64_t *>(vmeta + M_N_EVAL);
+                    const uint64_t t0 = (uint64_t)tile * (32u * P);
+                    full = t0 + lane_point<P>(lane, P - 1) < n_eval;
+                    if (!full) {
 #pragma unroll
                         for (int q = 0; q < P; ++q) {
                             if (t0 + lane_point<P>(lane, q) < n_eval) {
@@ -270,22 +280,37 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
                             }
                         }
                     }
-                    sacc[(g * 2) * 32 + lane] = k.s;
-                    sacc[(g * 2 + 1) * 32 + lane] = k.c;
                 }
+                if (full) {
+                    // the lane's P squared errors summed pairwise, then one
+                    // compensated add per tile
+                    float sq[P];
+#pragma unroll
+                    for (int q = 0; q < P; ++q) {
+                        const float d = pred.v[q] - y.v[q];
+                        sq[q] = d * d;
+                    }
+#pragma unroll
+                    for (int h = P / 2; h > 0; h /= 2)
+#pragma unroll
+                        for (int q = 0; q < h; ++q) sq[q] = sq[q] + sq[q + h];
+                    k.add(sq[0]);
+                }
+                sts_f32x2(kahan + 256u * g, k.s, k.c);
             }
-            if (tile == kNone) {
+            if (tile == kPrologue) {
                 __syncthreads();
-                tile = a.items[vmeta[24]].tile_begin + warp;
+                tile = vmeta[M_TILE_BEGIN] + warp;
             } else {
                 tile += nw;
             }
         }
         if (a.mode == MODE_MSE) {
             for (uint32_t g = 0; g < G; ++g) {
+                const float2 sc = lds_f32x2(kahan + 256u * g);
                 Kahan k;
-                k.s = sacc[(g * 2) * 32 + lane];
-                k.c = sacc[(g * 2 + 1) * 32 + lane];
+                k.s = sc.x;
+                k.c = sc.y;
                 const double s = warp_sum(k.value());
                 if (lane == 0) red[warp * kMaxProgsPerWarp + g] = s;
             }
@@ -305,12 +330,12 @@ __global__ void __launch_bounds__(kRegThreads, reg_min_blocks<PROF, P, OMIT>()) 
 }
 
 // ------------------------------------------------------------- launchers
-// Shared-memory layout (floats).  Block header: code | constants | meta (32
-// words) | cross-warp sums (kRegThreads/32 x 8 doubles).  Per warp: stacks
+// Shared-memory layout (floats).  Block header: code | constants | RegMeta |
+// cross-warp sums (kRegThreads/32 x 8 doubles).  Per warp: stacks
 // (per type) | Kahan state.
 void reg_layout(uint32_t code_words, uint32_t const_floats, const uint32_t *stack_depth, int P, int G,
                 uint32_t *stack_off, uint32_t *acc_off, uint32_t *region_floats, uint32_t *block_hdr_floats) {
-    *block_hdr_floats = align4r(code_words) + align4r(const_floats) + 32u + 2u * (kRegThreads / 32) * kMaxProgsPerWarp;
+    *block_hdr_floats = align4r(code_words) + align4r(const_floats) + kMetaWords + 2u * (kRegThreads / 32) * kMaxProgsPerWarp;
     uint32_t off = 0;
     for (int t = 0; t < N_STACKS; ++t) {
         stack_off[t] = off;

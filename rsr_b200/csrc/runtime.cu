@@ -517,8 +517,8 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
         for (uint32_t i = 0; i < n; ++i) {
             const EncodedProgram &E = enc[i];
             cw += path[i] <= -2 ? E.tape_code.size() : path[i] == -1 ? E.slot_code.size()
-                : gradient ? E.adj_code.size() : E.reg_code.size();
-            cf += E.consts.size();
+                : gradient ? E.adj_code.size() : E.reg_code.size() + 1;
+            cf += E.consts.size() + E.n_hoist;
         }
         P.code.reserve(cw);
         P.consts.reserve(cf);
@@ -555,6 +555,12 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
         part += d.n_parts;
         P.code.insert(P.code.end(), code.begin(), code.end());
         P.consts.insert(P.consts.end(), E.consts.begin(), E.consts.end());
+        if (!gradient && path[i] >= 0) {
+            // as the register kernel's block keeps it: its programs follow
+            // one another here, and are staged with one copy
+            P.code.push_back(K_STOP);
+            P.consts.resize(P.consts.size() + E.n_hoist, 0.0f);
+        }
         P.progs[li] = d;
         P.flops += (uint64_t)(gradient ? E.adj_flops_per_point : E.flops_per_point) * n_eval;
         P.program_points += n_eval;
@@ -627,7 +633,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             g.code_words = std::max(g.code_words, cw);
             g.const_floats = std::max(g.const_floats, cf);
             g.slots = std::max(g.slots, sl);
-            items.emplace_back(len_sum, WorkItem{j, k - j, 0, 0, 0, 0});
+            items.emplace_back(len_sum, WorkItem{j, k - j, 0, 0, 0, ds});
             j = k;
         }
         // register kernel: the tuned points per thread, halved while a block

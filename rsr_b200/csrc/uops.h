@@ -192,7 +192,7 @@ struct WorkItem {
     uint32_t tile_begin;
     uint32_t tile_end;
     uint32_t chunk;       // partial-sum slot offset within each program
-    uint32_t pad;
+    uint32_t dataset;     // of its programs (register kernel)
 };
 
 }  // namespace rsr
