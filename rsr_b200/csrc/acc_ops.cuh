@@ -80,13 +80,13 @@ template <int P, int W, int OP>
 __device__ __forceinline__ void apply_bin(Vf<P> *a, const Vf<P> *b) {
     if constexpr (OP == BIN_ADD) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) a[i] = a[i] + b[i];
+        for (int i = 0; i < W; ++i) a[i] = add2(a[i], b[i]);
     } else if constexpr (OP == BIN_SUB) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) a[i] = a[i] - b[i];
+        for (int i = 0; i < W; ++i) a[i] = sub2(a[i], b[i]);
     } else if constexpr (OP == BIN_RSUB) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) a[i] = b[i] - a[i];
+        for (int i = 0; i < W; ++i) a[i] = sub2(b[i], a[i]);
     } else if constexpr (OP == BIN_MUL) {
         a[0] = a[0] * b[0];
     } else if constexpr (OP == BIN_DIV) {
