@@ -138,20 +138,18 @@ static_assert(M_PROLOGUES == M_PROGS + 2 * (kMaxProgsPerWarp + 1) && M_Y_OFF == 
 // then one region per warp (spill stacks | Kahan state).
 // Blocks per SM each instance is compiled for (the register cap follows):
 // as many as its accumulators allow without spilling.
-// At four points per lane a fourth block (64 registers, a few bytes of
-// spill) pays for the F and F+V3 profiles (vector workload: 4.75 ms against
-// 5.14 ms at three blocks); F+V2+M2 spills more there and keeps three.  At
-// eight points, the F+V3 instances without the leaf-matrix mat-vec handlers
-// fit a third block (80 registers, 52 bytes of spill; vector workload 4.29
-// ms against 4.50 ms at two blocks); with those handlers they spill twice as
-// much and keep two.
+// At four points per lane a fourth block (64 registers, at most 12 bytes of
+// spill) pays for the F, F+V3 and F+V2+M2 profiles (2x2 matrix programs over 16
+// data sets 3.66 -> 3.63 ms a call against three blocks).  At eight points, F
+// and F+V3 fit a third (80 registers, up to 32 bytes of spill; 256 matrix
+// programs x 1M points 2.09 -> 2.00 ms against two, vector workload 2.76 -> 2.74
+// ms a call); F+V2+M2 would spill several accumulators there.
 template <int PROF, int P, int OMIT>
 constexpr int reg_min_blocks() {
     if constexpr (PROF == P_ALL) return P >= 4 ? 1 : 2;
     else if constexpr (PROF == P_FV3M3) return P >= 4 ? 2 : 3;
-    else if constexpr (PROF == P_FV2M2) return P >= 8 ? 2 : P >= 4 ? 3 : 4;
-    else if constexpr (PROF == P_FV3 && (OMIT & 2) != 0) return P >= 8 ? 3 : 4;
-    else return P >= 8 ? 2 : 4;
+    else if constexpr (PROF == P_FV2M2) return P >= 8 ? 2 : 4;
+    else return P >= 8 ? 3 : 4;
 }
 
 template <int PROF, int P, int OMIT>
