@@ -177,6 +177,8 @@ static constexpr int kGradSlotDoubles = 33;      // sse + 32 gradient sums
 static uint64_t round_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
 // Work items an SM of a plan whose profiles run as one launch each.
 static constexpr uint64_t kMergeItemsPerSm = 2;
+static uint64_t chunks_of(uint64_t n_eval) { return (n_eval + kChunkPoints - 1) / kChunkPoints; }
+
 static int log2_bucket(uint64_t n) {
     int b = 0;
     while ((1ull << (b + 1)) <= n) ++b;
@@ -195,8 +197,28 @@ static TuneChoice default_choice(int profile, uint64_t n_eval) {
     }
 }
 
-static TuneChoice choice_for(rsr_ctx *ctx, int profile, uint64_t n_eval) {
+// Fewer programs an item where a plan has few of them: an item costs its block
+// about a third of a program's run to stage, and about one item's time is left
+// at the end, so the best G is near sqrt(n_chunks / (3 * resident blocks)),
+// n_chunks being the plan's programs times their chunks.  Sums do not depend on
+// G.  Device time at 4 (F, matrix; vector from 64k points) or 2 (vector below)
+// programs an item -> by this rule: 64 scalar programs x 400 points 31 -> 16 us,
+// 256 x 400 32 -> 17, 2048 x 400 80 -> 53, 1024 x 8000 154 -> 98; 24 vector
+// programs x 100k 61 -> 37, 256 x 16,000 120 -> 80; 64 matrix programs x 100k
+// 140 -> 87.  At 4096 vector programs x 100k one program an item is 20% slower.
+// From 256k points on the chunks alone keep the SMs level, and an item's
+// programs share the features it reads: 8 matrix programs x 1M points 115 us at
+// 4, 130 at 1.
+static int programs_an_item(int G, int num_sms, uint64_t n_eval, uint64_t n_chunks) {
+    if (n_eval >= 262144) return G;
+    int g = 1;
+    while (g < G && n_chunks >= 6ull * 3ull * (uint64_t)num_sms * (uint64_t)(g * g)) g *= 2;
+    return g;
+}
+
+static TuneChoice choice_for(rsr_ctx *ctx, int profile, uint64_t n_eval, uint64_t n_chunks) {
     TuneChoice c = default_choice(profile, n_eval);
+    c.G = programs_an_item(c.G, ctx->num_sms, n_eval, n_chunks);
     auto it = ctx->tune.find({profile, log2_bucket(n_eval)});
     if (it != ctx->tune.end()) c = it->second;
     if (ctx->opts.points_per_thread > 0) c.P = ctx->opts.points_per_thread;
@@ -322,8 +344,8 @@ static void sort_by_key(std::vector<std::pair<uint64_t, uint32_t>> *v, std::vect
 // launch without them.  Not where the deepest program's stacks would cost the others points
 // per lane (end_plan halves P until a block fits) or the datasets' sizes ask
 // for different ones, so that no program's result depends on it.
-static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *S, uint32_t n, std::mutex *table_mu) {
-    auto items_of = [&](uint32_t i) { return (plan.datasets[S->prog_ds[i]].n_eval + kChunkPoints - 1) / kChunkPoints; };
+static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *S, uint32_t n, uint64_t n_chunks, std::mutex *table_mu) {
+    auto items_of = [&](uint32_t i) { return chunks_of(plan.datasets[S->prog_ds[i]].n_eval); };
     uint64_t total = 0;
     for (uint32_t i = 0; i < n; ++i) total += items_of(i);
     if (total > 8ull * kMergeItemsPerSm * (uint64_t)ctx->num_sms) return;  // even at 8 programs an item
@@ -356,19 +378,21 @@ static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *
             }
             if (!split) continue;
             TuneChoice c;
+            int full_g = 1;  // programs an item in a large plan: items of that size count
             {
                 std::unique_lock<std::mutex> lock;
                 if (table_mu) lock = std::unique_lock<std::mutex>(*table_mu);
-                c = choice_for(ctx, prof, hi);
+                c = choice_for(ctx, prof, hi, n_chunks);
+                full_g = choice_for(ctx, prof, hi, ~0ull).G;
                 bool same = true;
                 for (int b = log2_bucket(std::max<uint64_t>(lo, 1)); b <= log2_bucket(std::max<uint64_t>(hi, 1)); ++b) {
-                    const TuneChoice d = choice_for(ctx, prof, std::min(std::max(1ull << b, (unsigned long long)lo), (unsigned long long)hi));
+                    const TuneChoice d = choice_for(ctx, prof, std::min(std::max(1ull << b, (unsigned long long)lo), (unsigned long long)hi), n_chunks);
                     same = same && d.P == c.P && d.G == c.G;
                 }
                 if (!same) continue;
             }
             const uint64_t most = set < 0 ? (uint64_t)ctx->num_sms / 2 : kMergeItemsPerSm * (uint64_t)ctx->num_sms;
-            if (items > (uint64_t)c.G * most) continue;
+            if (items > (uint64_t)full_g * most) continue;
             if (reg_smem_bytes(cw * (uint32_t)c.G, cf * (uint32_t)c.G, depth, c.P, c.G) > kRegSmemBudget) continue;
             const int merged = prof + kRegPathStride * (cls + 3 * (int)omit);
             for (uint32_t i = 0; i < n; ++i)
@@ -493,7 +517,10 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
     for (uint32_t i = 0; i < n; ++i)
         if (S->rc[i] != RSR_OK) return fail(S->rc[i], "program " + std::to_string(i) + ": " + S->msg[i]);
     std::unique_lock<std::mutex> table_lock;
-    if (!gradient) merge_small_launches(ctx, P, S, n, table_mu);
+    uint64_t n_chunks = 0;  // of the register kernel's programs
+    for (uint32_t i = 0; i < n; ++i)
+        if (path[i] >= 0) n_chunks += chunks_of(P.datasets[prog_ds[i]].n_eval);
+    if (!gradient) merge_small_launches(ctx, P, S, n, n_chunks, table_mu);
     // group programs by (path, dataset), each group sorted by descending code length
     // (one 64-bit key per program: path, dataset, then longer code first and
     // the caller's order among equals, as a stable sort by those would give)
@@ -594,7 +621,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             uint64_t max_eval = 0;
             for (uint32_t j = li; j < end; ++j) max_eval = std::max(max_eval, P.datasets[P.progs[j].dataset].n_eval);
             if (table_mu) table_lock = std::unique_lock<std::mutex>(*table_mu);
-            TuneChoice c = choice_for(ctx, g.profile, max_eval);
+            TuneChoice c = choice_for(ctx, g.profile, max_eval, n_chunks);
             if (table_lock.owns_lock()) table_lock.unlock();
             g.P = c.P;
             g.G = c.G;
