@@ -94,14 +94,16 @@ class Clocks:
         self.device = device
         self.proc = None
         self.lines = []
+        self.first = threading.Event()
 
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.device), f"--query-gpu={self.FIELDS}",
-                                          "--format=csv,noheader,nounits", "-lms", "50"],
+                                          "--format=csv,noheader,nounits", "-lms", "20"],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
+            self.first.wait(5)  # nvidia-smi takes longer to start than a short timed region
         except FileNotFoundError:
             self.proc = None
         return self
@@ -109,6 +111,7 @@ class Clocks:
     def _read(self):
         for line in self.proc.stdout:
             self.lines.append(line.strip())
+            self.first.set()
 
     def __exit__(self, *a):
         if self.proc:
