@@ -201,7 +201,8 @@ static TuneChoice default_choice(int profile, uint64_t n_eval) {
 // about a third of a program's run to stage, and about one item's time is left
 // at the end, so the best G is near sqrt(n_chunks / (3 * resident blocks)),
 // n_chunks being the plan's programs times their chunks.  Sums do not depend on
-// G.  Device time at 4 (F, matrix; vector from 64k points) or 2 (vector below)
+// G: what they depend on, the points per lane, is chosen for the full G
+// (end_plan).  Device time at 4 (F, matrix; vector from 64k points) or 2 (vector below)
 // programs an item -> by this rule: 64 scalar programs x 400 points 31 -> 16 us,
 // 256 x 400 32 -> 17, 2048 x 400 80 -> 53, 1024 x 8000 154 -> 98; 24 vector
 // programs x 100k 61 -> 37, 256 x 16,000 120 -> 80; 64 matrix programs x 100k
@@ -378,7 +379,7 @@ static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *
             }
             if (!split) continue;
             TuneChoice c;
-            int full_g = 1;  // programs an item in a large plan: items of that size count
+            int full_g = 1;  // programs an item in a large plan: items of that size count, and have to fit
             {
                 std::unique_lock<std::mutex> lock;
                 if (table_mu) lock = std::unique_lock<std::mutex>(*table_mu);
@@ -393,7 +394,7 @@ static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *
             }
             const uint64_t most = set < 0 ? (uint64_t)ctx->num_sms / 2 : kMergeItemsPerSm * (uint64_t)ctx->num_sms;
             if (items > (uint64_t)full_g * most) continue;
-            if (reg_smem_bytes(cw * (uint32_t)c.G, cf * (uint32_t)c.G, depth, c.P, c.G) > kRegSmemBudget) continue;
+            if (reg_smem_bytes(cw * (uint32_t)full_g, cf * (uint32_t)full_g, depth, c.P, full_g) > kRegSmemBudget) continue;
             const int merged = prof + kRegPathStride * (cls + 3 * (int)omit);
             for (uint32_t i = 0; i < n; ++i)
                 if (member(i)) S->path[i] = merged;
@@ -612,6 +613,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             for (uint32_t j = li; j < end; ++j) g.omit &= adj_omit[order[j]];
         }
         g.item_begin = (uint32_t)P.items.size();
+        int full_g = 1;  // register kernel: programs an item in a large plan
         if (g.kind == 3) {
             g.G = 1;
             g.P = adj_path_p(pth);
@@ -622,6 +624,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             for (uint32_t j = li; j < end; ++j) max_eval = std::max(max_eval, P.datasets[P.progs[j].dataset].n_eval);
             if (table_mu) table_lock = std::unique_lock<std::mutex>(*table_mu);
             TuneChoice c = choice_for(ctx, g.profile, max_eval, n_chunks);
+            full_g = choice_for(ctx, g.profile, max_eval, ~0ull).G;
             if (table_lock.owns_lock()) table_lock.unlock();
             g.P = c.P;
             g.G = c.G;
@@ -664,10 +667,23 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             j = k;
         }
         // register kernel: the tuned points per thread, halved while a block
-        // would not fit
-        if (g.kind == 1)
-            while (g.P > 2 && reg_smem_bytes(g.code_words, g.const_floats, g.stack_depth, g.P, g.G) > kRegSmemBudget)
+        // would not fit.  They set the order of a program's sums, so the block
+        // is that of a large plan's items (full_g programs), whatever G is here.
+        if (g.kind == 1) {
+            uint32_t code_words = 0, const_floats = 0;
+            for (uint32_t q = li; q < end;) {
+                uint32_t cw = 0, cf = 0;
+                const uint32_t first = q, ds = P.progs[q].dataset;
+                for (; q < end && q - first < (uint32_t)full_g && P.progs[q].dataset == ds; ++q) {
+                    cw += P.progs[q].uop_len + 1;
+                    cf += P.progs[q].n_consts + P.progs[q].n_tape;
+                }
+                code_words = std::max(code_words, cw);
+                const_floats = std::max(const_floats, cf);
+            }
+            while (g.P > 2 && reg_smem_bytes(code_words, const_floats, g.stack_depth, g.P, full_g) > kRegSmemBudget)
                 g.P >>= 1;
+        }
         // points per thread of the slot-file kernel: largest that fits the smem budget
         if (g.kind == 0) {
             int Pp = 4;
