@@ -53,7 +53,7 @@ template <int P>
 struct RevIO : AccIO<P> {
     uint32_t tm;            // tensor-memory tape: this warp's lanes, column 0
     uint32_t gacc;          // shared-memory address of this lane's f32 gradient sums, one row of 32 a parameter
-    uint32_t valid;         // bit q: value q of the lane is a counted point
+    uint32_t valid;         // counted_points of the lane and tile
     // a tape reference (uops.h, kTapeRefX) of a value of W components: tape
     // slots, or the features or constants the forward value was loaded from
     template <int W>
@@ -90,7 +90,8 @@ struct RevIO : AccIO<P> {
     }
     // Adds the lane's counted points of g, in order, to the sum of flat
     // parameter k (points past the dataset's end may carry 0*inf = NaN
-    // adjoints); parameters from kAdjParams on share a row nobody reads.
+    // adjoints); parameters from kAdjParams on share a row nobody reads.  The
+    // branch is on the tile being cut off, which is so for the whole warp.
     // One asm statement, so that nvcc sees no branch here: with one it kept
     // copies of the adjoints for the merge behind it, and the reverse loop
     // moved accumulators in every entry (32 of 36 instructions of one that
@@ -105,8 +106,8 @@ struct RevIO : AccIO<P> {
                          ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "r"(valid) : "memory");
         } else if constexpr (P == 4) {
             asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
-                         "mov.f32 s, 0f00000000;\nsetp.ne.u32 p, %5, 15;\n@p bra PART;\n"
-                         "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\nbra DONE;\n"
+                         "mov.f32 s, 0f00000000;\nsetp.gt.u32 p, %5, 15;\n@p bra.uni PART;\n"
+                         "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\nbra.uni DONE;\n"
                          "PART:\n"
                          "and.b32 b, %5, 1;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %1;\n"
                          "and.b32 b, %5, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
@@ -116,9 +117,9 @@ struct RevIO : AccIO<P> {
                          ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "r"(valid) : "memory");
         } else {
             asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
-                         "mov.f32 s, 0f00000000;\nsetp.ne.u32 p, %9, 255;\n@p bra PART;\n"
+                         "mov.f32 s, 0f00000000;\nsetp.gt.u32 p, %9, 255;\n@p bra.uni PART;\n"
                          "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\n"
-                         "add.rn.f32 s, s, %5;\nadd.rn.f32 s, s, %6;\nadd.rn.f32 s, s, %7;\nadd.rn.f32 s, s, %8;\nbra DONE;\n"
+                         "add.rn.f32 s, s, %5;\nadd.rn.f32 s, s, %6;\nadd.rn.f32 s, s, %7;\nadd.rn.f32 s, s, %8;\nbra.uni DONE;\n"
                          "PART:\n"
                          "and.b32 b, %9, 1;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %1;\n"
                          "and.b32 b, %9, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
@@ -705,12 +706,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
                 const uint64_t t0 = (uint64_t)tile * (32u * P);
                 const uint64_t p0 = t0 + lane_point<P>(lane, 0);
                 io.xl = opaque(ds.x + p0);
-                uint32_t valid = (1u << P) - 1u;
-                if (t0 + 32u * P > ds.n_eval) {
-                    valid = 0;
-#pragma unroll
-                    for (int q = 0; q < P; ++q) valid |= (t0 + lane_point<P>(lane, q) < ds.n_eval ? 1u : 0u) << q;
-                }
+                const uint32_t valid = counted_points<P>(lane, t0, ds.n_eval);
                 io.valid = valid;
                 Acc<PROF, P> acc;
                 run_forward<PROF, P, OMIT>(acc, io, fwd);

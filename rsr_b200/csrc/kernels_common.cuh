@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 
+#include "lane_layout.h"
 #include "uops.h"
 #include "vm_ops.cuh"
 
@@ -128,24 +129,6 @@ __device__ __forceinline__ void store_pts(float *p, const Vf<P> &v, uint64_t fir
 #pragma unroll
     for (int k = 0; k < P; ++k)
         if (first + k < limit) p[k] = v.v[k];
-}
-
-// ------------------------------------------------ interleaved lane layout
-// The register kernels give lane l of a warp the points of a 32*P-point
-// tile in runs of at most four: P <= 4, points l*P .. l*P+P-1; P = 8, points
-// 4l .. 4l+3 and 128+4l .. 128+4l+3.  Each 16-byte access of the warp then
-// covers 512 contiguous bytes -- four L1 wavefronts for a global load, no
-// bank conflict for shared memory -- where eight consecutive points a lane
-// would take eight (two lanes 32 bytes apart share a 128-byte line or a bank).
-// Per-lane values in shared memory use the same layout in blocks of 32*P
-// floats: [P/4 runs][32 lanes][4] (P >= 4), [32 lanes][P] below.
-template <int P>
-constexpr int kLaneRun = P < 4 ? P : 4;
-
-// Offset of value q of `lane` from the start of its tile (or block).
-template <int P>
-__host__ __device__ __forceinline__ constexpr uint32_t lane_point(int lane, int q) {
-    return (uint32_t)((q / kLaneRun<P>) * 32 * kLaneRun<P> + lane * kLaneRun<P> + q % kLaneRun<P>);
 }
 
 // Loads a lane's P values; p points at its first (tile start + lane_point(lane, 0)).
