@@ -197,29 +197,41 @@ static TuneChoice default_choice(int profile, uint64_t n_eval) {
     }
 }
 
+// The register kernel's share of a plan: its programs, and their chunks (a
+// program's data set cut into parts, summed over the programs).
+struct PlanSize {
+    uint64_t programs = 0, chunks = 0;
+};
+static constexpr PlanSize kLargePlan{1, ~0ull};
+
 // Fewer programs an item where a plan has few of them: an item costs its block
 // about a third of a program's run to stage, and about one item's time is left
-// at the end, so the best G is near sqrt(n_chunks / (3 * resident blocks)),
-// n_chunks being the plan's programs times their chunks.  Sums do not depend on
-// G: what they depend on, the points per lane, is chosen for the full G
-// (end_plan).  Device time at 4 (F, matrix; vector from 64k points) or 2 (vector below)
-// programs an item -> by this rule: 64 scalar programs x 400 points 31 -> 16 us,
-// 256 x 400 32 -> 17, 2048 x 400 80 -> 53, 1024 x 8000 154 -> 98; 24 vector
-// programs x 100k 61 -> 37, 256 x 16,000 120 -> 80; 64 matrix programs x 100k
-// 140 -> 87.  At 4096 vector programs x 100k one program an item is 20% slower.
-// From 256k points on the chunks alone keep the SMs level, and an item's
-// programs share the features it reads: 8 matrix programs x 1M points 115 us at
-// 4, 130 at 1.
-static int programs_an_item(int G, int num_sms, uint64_t n_eval, uint64_t n_chunks) {
-    if (n_eval >= 262144) return G;
+// at the end, so the best G is near sqrt(chunks / (3 * resident blocks)).  Sums
+// do not depend on G: what they depend on, the points per lane, is chosen for
+// the full G (end_plan).  Device time at 4 (F, matrix; vector from 64k points) or
+// 2 (vector below) programs an item -> by this rule: 64 scalar programs x 400
+// points 31 -> 16 us, 256 x 400 32 -> 17, 2048 x 400 80 -> 53, 1024 x 8000 154 ->
+// 98; 24 vector programs x 100k 61 -> 37, 256 x 16,000 120 -> 80; 64 matrix
+// programs x 100k 140 -> 87; x 262,144 points: 4 vector programs 51 -> 27, 4 scalar
+// 49 -> 33, 8 matrix 90 -> 50, 4 2x2 matrix 90 -> 46 and 64 of them 377 -> 290.  At
+// 4096 vector programs x 100k one program an item is 20% slower.
+// F+V3 with data sets of one and a half chunks an SM or more (on average over
+// the plan) keeps the full G: a group of G programs fills the device by itself, and
+// shares the features it reads.  On 1M points 4 vector programs take 73 us at 4
+// an item and 81 at 1, 8 matrix programs 120 and 139; below, on 900k points, 4
+// vector programs 69 and 68, 8 matrix programs 117 and 112, on 600k 59 and 47, 101
+// and 84.  The other profiles do not gain by it: on 1M points 8 scalar programs
+// take 116 us at 4 an item and 96 at 1, 8 2x2 matrix programs 227 and 163.
+static int programs_an_item(int profile, int G, int num_sms, PlanSize size) {
+    if (profile == P_FV3 && size.chunks >= 3ull * (uint64_t)num_sms * size.programs / 2) return G;
     int g = 1;
-    while (g < G && n_chunks >= 6ull * 3ull * (uint64_t)num_sms * (uint64_t)(g * g)) g *= 2;
+    while (g < G && size.chunks >= 6ull * 3ull * (uint64_t)num_sms * (uint64_t)(g * g)) g *= 2;
     return g;
 }
 
-static TuneChoice choice_for(rsr_ctx *ctx, int profile, uint64_t n_eval, uint64_t n_chunks) {
+static TuneChoice choice_for(rsr_ctx *ctx, int profile, uint64_t n_eval, PlanSize size) {
     TuneChoice c = default_choice(profile, n_eval);
-    c.G = programs_an_item(c.G, ctx->num_sms, n_eval, n_chunks);
+    c.G = programs_an_item(profile, c.G, ctx->num_sms, size);
     auto it = ctx->tune.find({profile, log2_bucket(n_eval)});
     if (it != ctx->tune.end()) c = it->second;
     if (ctx->opts.points_per_thread > 0) c.P = ctx->opts.points_per_thread;
@@ -345,7 +357,7 @@ static void sort_by_key(std::vector<std::pair<uint64_t, uint32_t>> *v, std::vect
 // launch without them.  Not where the deepest program's stacks would cost the others points
 // per lane (end_plan halves P until a block fits) or the datasets' sizes ask
 // for different ones, so that no program's result depends on it.
-static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *S, uint32_t n, uint64_t n_chunks, std::mutex *table_mu) {
+static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *S, uint32_t n, PlanSize size, std::mutex *table_mu) {
     auto items_of = [&](uint32_t i) { return chunks_of(plan.datasets[S->prog_ds[i]].n_eval); };
     uint64_t total = 0;
     for (uint32_t i = 0; i < n; ++i) total += items_of(i);
@@ -383,11 +395,11 @@ static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *
             {
                 std::unique_lock<std::mutex> lock;
                 if (table_mu) lock = std::unique_lock<std::mutex>(*table_mu);
-                c = choice_for(ctx, prof, hi, n_chunks);
-                full_g = choice_for(ctx, prof, hi, ~0ull).G;
+                c = choice_for(ctx, prof, hi, size);
+                full_g = choice_for(ctx, prof, hi, kLargePlan).G;
                 bool same = true;
                 for (int b = log2_bucket(std::max<uint64_t>(lo, 1)); b <= log2_bucket(std::max<uint64_t>(hi, 1)); ++b) {
-                    const TuneChoice d = choice_for(ctx, prof, std::min(std::max(1ull << b, (unsigned long long)lo), (unsigned long long)hi), n_chunks);
+                    const TuneChoice d = choice_for(ctx, prof, std::min(std::max(1ull << b, (unsigned long long)lo), (unsigned long long)hi), size);
                     same = same && d.P == c.P && d.G == c.G;
                 }
                 if (!same) continue;
@@ -518,10 +530,13 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
     for (uint32_t i = 0; i < n; ++i)
         if (S->rc[i] != RSR_OK) return fail(S->rc[i], "program " + std::to_string(i) + ": " + S->msg[i]);
     std::unique_lock<std::mutex> table_lock;
-    uint64_t n_chunks = 0;  // of the register kernel's programs
+    PlanSize size;
     for (uint32_t i = 0; i < n; ++i)
-        if (path[i] >= 0) n_chunks += chunks_of(P.datasets[prog_ds[i]].n_eval);
-    if (!gradient) merge_small_launches(ctx, P, S, n, n_chunks, table_mu);
+        if (path[i] >= 0) {
+            ++size.programs;
+            size.chunks += chunks_of(P.datasets[prog_ds[i]].n_eval);
+        }
+    if (!gradient) merge_small_launches(ctx, P, S, n, size, table_mu);
     // group programs by (path, dataset), each group sorted by descending code length
     // (one 64-bit key per program: path, dataset, then longer code first and
     // the caller's order among equals, as a stable sort by those would give)
@@ -623,8 +638,8 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             uint64_t max_eval = 0;
             for (uint32_t j = li; j < end; ++j) max_eval = std::max(max_eval, P.datasets[P.progs[j].dataset].n_eval);
             if (table_mu) table_lock = std::unique_lock<std::mutex>(*table_mu);
-            TuneChoice c = choice_for(ctx, g.profile, max_eval, n_chunks);
-            full_g = choice_for(ctx, g.profile, max_eval, ~0ull).G;
+            TuneChoice c = choice_for(ctx, g.profile, max_eval, size);
+            full_g = choice_for(ctx, g.profile, max_eval, kLargePlan).G;
             if (table_lock.owns_lock()) table_lock.unlock();
             g.P = c.P;
             g.G = c.G;
