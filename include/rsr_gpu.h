@@ -134,6 +134,8 @@ RSR_API int rsr_dataset_subset(rsr_ctx *ctx, rsr_dataset src, uint64_t target_sa
 /* A resident dataset back in the AoSoA layout: feature_flat
  * [num_batches*num_features*8], target_batches [num_batches*8]. */
 RSR_API int rsr_dataset_download(rsr_ctx *ctx, rsr_dataset ds, float *feature_flat, float *target_batches);
+/* Frees a dataset; with the context's last one go the buffers that a fit left
+ * for the next (rsr_fit_lbfgs). */
 RSR_API int rsr_dataset_release(rsr_ctx *ctx, rsr_dataset ds);
 RSR_API int rsr_dataset_info(rsr_ctx *ctx, rsr_dataset ds, uint32_t *num_features, uint64_t *num_batches,
                      uint64_t *num_samples);
@@ -201,7 +203,8 @@ typedef struct rsr_fit_stats {
  * parameters, Armijo backtracking c1 = 1e-4 with up to 11 halvings, stop at
  * |grad| < 1e-5), gradients from the adjoint kernel, line-search MSEs from
  * the register kernel.  params_out (same layout as pop->params) receives the
- * fitted constants, mse_out[i] the final fitness of program i. */
+ * fitted constants, mse_out[i] the final fitness of program i.  The context
+ * keeps up to 256 MB of device and pinned buffers for its next fit. */
 RSR_API int rsr_fit_lbfgs(rsr_ctx *ctx, const rsr_population *pop, rsr_dataset ds, const rsr_dataset *ds_per_program,
                           uint32_t max_iterations, float *params_out, float *mse_out, rsr_fit_stats *stats);
 

@@ -455,8 +455,9 @@ extern "C" int rsr_fit_lbfgs(rsr_ctx *ctx, const rsr_population *pop, rsr_datase
     if (!ctx || !pop || !params_out || !mse_out) return fail(RSR_EINVAL, "null argument");
     std::lock_guard<std::mutex> lk(ctx->mu);
     cudaSetDevice(ctx->device);
-    // The buffers stay for the context's next fit, up to a size: allocating
-    // and freeing them (pinned memory above all) took 1 to 5 ms a call.
+    // The buffers stay for the context's next fit, up to a size and until its
+    // last data set is released (rsr_dataset_release): allocating and freeing
+    // them (pinned memory above all) took 1 to 5 ms a call.
     constexpr size_t kKeepBytes = (size_t)256 << 20;
     if (!ctx->fit) ctx->fit = std::make_unique<FitWorkspace>();
     const int rc = fit_population(ctx, pop, dsp, ds, max_iterations, ctx->stream, nullptr, nullptr, ctx->fit.get(),

@@ -1414,6 +1414,7 @@ int rsr_dataset_release(rsr_ctx *ctx, rsr_dataset ds) {
     cudaFree(it->second->y);
     ctx->mem_in_use -= it->second->bytes;
     ctx->datasets.erase(it);
+    if (ctx->datasets.empty()) ctx->fit.reset();  // nothing left to fit to: a fit's buffers go too
     return RSR_OK;
 }
 
