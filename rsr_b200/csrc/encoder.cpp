@@ -1071,7 +1071,7 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
         std::vector<Node> &kept = tls.hoisted_nodes;
         hoist.clear();
         kept.clear();
-        uint32_t types = 0, n_hoist = 0;
+        uint32_t types = 0, n_hoist = 0, hoisted_flops = 0;
         bool ok = true;
         if (forms & FORM_HOIST) {
             // the largest constant subtrees: those a node that is not
@@ -1088,6 +1088,8 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
             n_hoist = 0;
         }
         if (!hoist.empty()) {
+            for (size_t i = 0; i < nodes.size(); ++i)
+                if (live[i] && nodes[i].is_const) hoisted_flops += op_sig(nodes[i].opcode).flops;
             AccEmitter em(nodes);
             ok = em.analyze(root);
             for (size_t h = 0; ok && h < hoist.size(); ++h) {
@@ -1121,6 +1123,7 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
             if (E.profile >= 0) {
                 E.main_off = (uint32_t)E.reg_code.size();
                 E.n_hoist = n_hoist;
+                E.hoisted_flops = hoisted_flops;
                 E.reg_code.insert(E.reg_code.end(), em.code.begin(), em.code.end());
             }
         }

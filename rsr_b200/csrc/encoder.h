@@ -30,7 +30,7 @@ struct EncodedProgram {
     // common
     uint32_t n_params = 0;
     std::vector<float> consts;            // flat parameters (kernel constant pool)
-    uint32_t flops_per_point = 0;         // incl. MSE epilogue
+    uint32_t flops_per_point = 0;         // the program's operations, incl. MSE epilogue
     uint32_t adj_flops_per_point = 0;     // forward + reverse sweep (adjoint kernel), incl. epilogues
     bool differentiable = true;
     bool result_zero = false;             // stack_f[0] is never written
@@ -45,6 +45,7 @@ struct EncodedProgram {
     std::vector<uint32_t> reg_code;
     uint32_t main_off = 0;                // first word of the main program (FORM_HOIST: behind the prologue)
     uint32_t n_hoist = 0;                 // floats the prologue adds to the constants
+    uint32_t hoisted_flops = 0;           // operations of flops_per_point that the prologue runs once an item
     // adjoint (slot form with one slot range per value, never reused)
     std::vector<uint32_t> tape_code;      // 2 header words + 5 words per live node
     uint32_t n_tape_val = 0, n_tape_adj = 0;  // scalar value / adjoint slots

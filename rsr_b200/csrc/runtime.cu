@@ -605,7 +605,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
             P.consts.resize(P.consts.size() + E.n_hoist, 0.0f);
         }
         P.progs[li] = d;
-        P.flops += (uint64_t)(gradient ? E.adj_flops_per_point : E.flops_per_point) * n_eval;
+        P.flops += (uint64_t)(gradient ? E.adj_flops_per_point : E.flops_per_point - E.hoisted_flops) * n_eval;
         P.program_points += n_eval;
     }
     P.n_partials = part * (gradient ? kGradSlotDoubles : 1);
@@ -787,7 +787,7 @@ static int end_plan(rsr_ctx *ctx, const rsr_population &pop, Plan *plan, EncodeS
         for (uint32_t q = li; q < end; ++q) {
             const EncodedProgram &E = enc[order[q]];
             const uint64_t ne = P.datasets[P.progs[q].dataset].n_eval;
-            g.flops += (uint64_t)(gradient ? E.adj_flops_per_point : E.flops_per_point) * ne;
+            g.flops += (uint64_t)(gradient ? E.adj_flops_per_point : E.flops_per_point - E.hoisted_flops) * ne;
             g.program_points += ne;
         }
         P.groups.push_back(g);

@@ -117,7 +117,7 @@ struct Group {
     mutable size_t smem = 0;
     mutable uint32_t warps_per_block = 0;
     mutable uint32_t tmem_cols = 0;     // register adjoint: tensor-memory columns of a warp's tape
-    uint64_t flops = 0;           // algorithmic FP32 lane-ops of one run
+    uint64_t flops = 0;           // FP32 lane-ops of one run at every point (not a prologue's)
     uint64_t program_points = 0;
     uint64_t item_work = 0;       // code length x tiles of the group's longest item
 };
@@ -139,7 +139,7 @@ struct Plan {
     bool one_part = false;                  // MODE_MSE: every program has one part and runs on a register kernel
     int mode = MODE_MSE;
     uint64_t points_stride = 0;
-    uint64_t flops = 0;                     // algorithmic lane-ops of one run
+    uint64_t flops = 0;                     // lane-ops of one run, as the groups count them
     uint64_t program_points = 0;
     uint32_t n_plain = 0, n_reg = 0;
 
