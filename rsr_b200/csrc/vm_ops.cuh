@@ -158,11 +158,13 @@ template <int P> __device__ __forceinline__ Vf<P> vlog(const Vf<P> &a) { Vf<P> r
 // apart.  Inside the range: Newton's method on the hardware's reciprocal (square
 // root), then Markstein's correction by the exact FMA remainder (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34(1), 1990).  Checked against sqrtf for every float of the
-// range, and against / for every pair of mantissas (2^46) and for 6e10 pairs
-// with random exponents in it; the FMA steps run on two values at a time.
-// Before they did:  4096 vector programs x 100k points 2.90 -> 2.78 ms, 2048 2x2 matrix
-// programs with inverses 2.38 -> 2.19 ms, vector gradients 11.7 -> 11.4 ms.
+// IBM J. Res. Dev. 34(1), 1990), the FMA steps on two values at a time.
+// tests/test_div_sqrt_range.py compares them with the IEEE results bit for bit:
+// roots of every mantissa at exponents of both parities and at both ends,
+// quotients by every mantissa with random dividends, and 2.6 million quotients
+// next to the middle between two floats.  With the shared test, before the FMA
+// steps were paired: 4096 vector programs x 100k points 2.90 -> 2.78 ms, 2048 2x2
+// matrix programs with inverses 2.38 -> 2.19 ms, vector gradients 11.7 -> 11.4 ms.
 __device__ __forceinline__ float min_nan3(float a, float b, float c) {
     float r;
     asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
