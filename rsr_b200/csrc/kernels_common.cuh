@@ -28,7 +28,6 @@ struct LaunchArgs {
     uint32_t *item_counter;   // persistent kernels: next work item; 0 before and after a launch
     float *mse_out;           // register kernels, when every program has one part: the epilogue's
     float *grad_out;          // results, written by the item's block (no finalize launch); else null
-    uint32_t *status;         // sticky error flags (bit 0: bad micro-op)
     const uint8_t *active;    // optional per-program mask (launch order): 0 = skip
     const uint32_t *run_if;   // optional: the launch does nothing when *run_if == 0 (device-side
                               // loops whose later rounds may have no work, e.g. line searches)

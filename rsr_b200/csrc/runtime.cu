@@ -885,21 +885,19 @@ int upload_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t st
     return RSR_OK;
 }
 
-// Blocks per SM of a register or register-adjoint instance at a shared-memory
-// size, from the occupancy API once per (device, instance, size): the query
-// costs the host more than the launch it sizes.
-static int blocks_per_sm(int device, int kind, int profile, int P, unsigned omit, size_t smem) {
+// Blocks per SM of a register-kernel instance at a shared-memory size, from the
+// occupancy API once per (device, instance, size): the query costs the host
+// more than the launch it sizes.
+static int blocks_per_sm(int device, int profile, int P, unsigned omit, size_t smem) {
     static std::mutex mu;
     static std::unordered_map<uint64_t, int> cache;
-    const uint64_t key = ((uint64_t)(device & 255) << 56) | ((uint64_t)(kind & 3) << 54) |
-                         ((uint64_t)(profile & 7) << 51) | ((uint64_t)(P & 15) << 47) | ((uint64_t)(omit & 3) << 45) |
-                         (uint64_t)(smem & ((1ull << 45) - 1));
+    const uint64_t key = ((uint64_t)(device & 255) << 56) | ((uint64_t)(profile & 7) << 51) | ((uint64_t)(P & 15) << 47) |
+                         ((uint64_t)(omit & 3) << 45) | (uint64_t)(smem & ((1ull << 45) - 1));
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if (it != cache.end()) return it->second;
     }
-    (void)kind;
     const int n = reg_max_blocks_per_sm(profile, P, omit, smem);
     if (n > 0) {
         std::lock_guard<std::mutex> lk(mu);
@@ -991,7 +989,7 @@ int enqueue_plan(rsr_ctx *ctx, const Plan &plan, DevicePlan *dev, cudaStream_t s
             reg_layout(g.code_words, g.const_floats, g.stack_depth, g.P, g.G, a.stack_off, &a.acc_off, &a.region_floats,
                        &a.block_hdr_floats);
             const size_t smem = ((size_t)a.block_hdr_floats + (size_t)a.region_floats * (kRegThreads / 32)) * 4u;
-            int bps = std::max(1, blocks_per_sm(ctx->device, 1, g.profile, g.P, g.omit, smem));
+            int bps = std::max(1, blocks_per_sm(ctx->device, g.profile, g.P, g.omit, smem));
             uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)bps * ctx->num_sms, g.n_items);
             g.grid = std::max(1u, grid);
             g.smem = smem;
@@ -1088,7 +1086,6 @@ static int fetch_results(rsr_ctx *ctx, const Plan &plan, DevicePlan &dev, cudaSt
         if (mse_out) mse_out[plan.orig[li]] = tmp[li];
         if (grad_out && plan.gradient) memcpy(grad_out + (size_t)plan.orig[li] * 32, tmp + n + li * 32, 32 * sizeof(float));
     }
-    (void)ctx;
     return RSR_OK;
 }
 
