@@ -149,11 +149,11 @@ __device__ __forceinline__ void unary_prefix(Vf<P> *A, const AccIO<P> &io, int t
 }
 
 // Ends the handler of kind K: an empty statement that differs from every
-// other handler's.  Without it nvcc moves the tail that handlers have in
-// common (the parameter sums of a constant operand, say) into one block
-// behind the switch, and every micro-op, whatever its kind, then pays the
-// copies of the accumulators into that block's registers: 24 of the 36
-// instructions of an F+V3 reverse entry that does nothing.
+// other handler's, so that handlers which end alike (in the parameter sums of a
+// constant operand, say) are not joined behind the switch, with copies of the
+// accumulators for every kind.  Without it -> with it: gradients of 256 matrix
+// programs x 1M points 8.98 -> 8.76 ms, 8192 2x2 matrix programs over 16 data sets
+// 8.05 -> 7.71; vector programs are even (2.30 ms, gradients 10.63 -> 10.67).
 template <int K>
 __device__ __forceinline__ void handler_end() {
     asm volatile("// %0" ::"n"(K));

@@ -58,7 +58,7 @@ int reg_max_blocks_per_sm(int profile, int P, unsigned omit, size_t smem);
 bool adj_supported(int profile);
 int adj_max_p(int profile);
 // floats of a warp's shared-memory region for a program (stacks, shared by
-// the adjoint stacks | gradient sums | Kahan state), and its stack depths
+// the adjoint stacks | gradient sums | squared errors), and its stack depths
 // packed for ProgDesc
 uint32_t adj_warp_floats(const uint32_t *stack_depth, int P, uint32_t n_params);
 uint32_t adj_pack_depth(const uint32_t *stack_depth);

@@ -8,7 +8,7 @@
 //   forward  the accumulator form (acc_ops.cuh) with a load after a PUSH
 //            fused into the PUSH and every PUSH to its own stack slot; the
 //            forward values the reverse rules read go to a per-warp tape in
-//            shared memory, stored by the op's own entry (before or after
+//            tensor memory, stored by the op's own entry (before or after
 //            the op) or by a TAPE micro-op;
 //   seed     G_F = 2 (pred - y) on counted points (evaluator.rs:207);
 //   reverse  the reverse entries (uops.h, kAdjHeaderWords): each maps the
@@ -92,10 +92,10 @@ struct RevIO : AccIO<P> {
     // parameter k (points past the dataset's end may carry 0*inf = NaN
     // adjoints); parameters from kAdjParams on share a row nobody reads.  The
     // branch is on the tile being cut off, which is so for the whole warp.
-    // One asm statement, so that nvcc sees no branch here: with one it kept
-    // copies of the adjoints for the merge behind it, and the reverse loop
-    // moved accumulators in every entry (32 of 36 instructions of one that
-    // does nothing).
+    // One asm statement, so that nvcc has no branch here to keep the adjoints
+    // apart for: gradients of 4096 vector programs x 100k points 10.99 ms with
+    // the sum as a loop in C++, 10.67 so (256 matrix programs x 1M points 8.75
+    // and 8.76).
     __device__ __forceinline__ void grad_add(uint32_t k, const Vf<P> &g) const {
         const uint32_t row = gacc + 128u * min(k, kAdjParams);
         if constexpr (P == 2) {
@@ -620,10 +620,10 @@ __device__ __forceinline__ void run_reverse(Acc<PROF, P> &g, const RevIO<P> &io,
 // Warps of a block of instance (PROF, P), one block per SM: a multiple of
 // 4, at most 16.  More warps than the instance's registers allow unspilled
 // pay: the extra warps hide more of the dispatch latency than the spill
-// costs.  F+V3 at 8 points per lane: 168 registers at 12 warps, 128 with
-// ~250 bytes of spill at 16 (vector workload gradient 17.7 ms against 22.4
-// ms); F+V2+M2 and F+V3+M3 at 4 points likewise at 16 and 12 warps (matrix
-// workload 17.0 against 18.7 ms).
+// costs.  F+V3 at 8 points per lane: 168 registers at 12 warps, 128 with 80 to
+// 124 bytes of spill stores at 16 (gradients of 4096 vector programs x 100k
+// points 14.02 ms and 10.67, of 256 matrix programs x 1M points 11.77 and 8.76).
+// F+V3+M3 at 4 points spills 1 KB at 12 already and stays there.
 template <int PROF, int P>
 __host__ __device__ constexpr int adj_warps() {
     if constexpr (PROF == P_FV3M3) return P >= 4 ? 12 : 16;

@@ -136,14 +136,14 @@ static_assert(M_PROLOGUES == M_PROGS + 2 * (kMaxProgsPerWarp + 1) && M_Y_OFF == 
 //
 // Shared memory: block header (code | constants | meta | cross-warp sums)
 // then one region per warp (spill stacks | Kahan state).
-// Blocks per SM each instance is compiled for (the register cap follows):
-// as many as its accumulators allow without spilling.
-// At four points per lane a fourth block (64 registers, at most 12 bytes of
-// spill) pays for the F, F+V3 and F+V2+M2 profiles (2x2 matrix programs over 16
-// data sets 3.66 -> 3.63 ms a call against three blocks).  At eight points, F
-// and F+V3 fit a third (80 registers, up to 32 bytes of spill; 256 matrix
-// programs x 1M points 2.09 -> 2.00 ms against two, vector workload 2.76 -> 2.74
-// ms a call); F+V2+M2 would spill several accumulators there.
+// Blocks per SM each instance is compiled for (the register cap follows): as
+// many as its accumulators allow, with a few bytes of spill where one more block
+// is worth them.  Device time against one block fewer: F and F+V3 at eight
+// points, a third (80 registers, up to 32 bytes of spill stores), 4096 vector
+// programs x 100k points 2.68 -> 2.30 ms, 256 matrix programs x 1M points 2.12 ->
+// 1.92, 1024 scalar programs x 100k points 0.87 -> 0.79; F+V2+M2 would spill several
+// accumulators there.  F+V2+M2 at four points, a fourth (64 registers, 12 bytes):
+// 8192 programs over 16 data sets 7.73 -> 7.71, as much as that measurement can tell.
 template <int PROF, int P, int OMIT>
 constexpr int reg_min_blocks() {
     if constexpr (PROF == P_ALL) return P >= 4 ? 1 : 2;

@@ -147,9 +147,9 @@ static constexpr size_t kGradTapeBudget = 80 * 1024;
 // number of its launches in a gradient plan.
 static constexpr size_t kAdjRegionBudget = 200 * 1024;
 static constexpr int kAdjPathBase = 0;
-// Points per work-item chunk (all P).  8192 measured slower on every kernel
-// (vector register 4.32 ms against 4.30, matrix register 4.84 against 4.69,
-// vector adjoint 6.68 against 5.90): coarser items balance worse.
+// Points per work-item chunk (all P).  8192 measured slower on every kernel, when
+// they took about twice as long as now (vector register 4.32 ms against 4.30,
+// matrix register 4.84 against 4.69): coarser items balance worse.
 static constexpr uint64_t kChunkPoints = kPartPoints;
 // Work items of the register adjoint cover several parts: its block is the
 // SM's only one, and between items the SM waits for the next item's code
@@ -188,7 +188,7 @@ static int log2_bucket(uint64_t n) {
 // Default launch shape of the register kernel per profile: points per
 // thread and programs per warp.  F+V3 on 64k points or more takes the shape
 // the autotuner picks for the 100k-point vector workload (8 points per lane,
-// 4 programs per item: 4.28 ms against 4.56 ms at 4 and 2).
+// 4 programs per item: 2.30 ms against 2.63 ms at 4 and 2).
 static TuneChoice default_choice(int profile, uint64_t n_eval) {
     switch (profile) {
         case P_F: return {8, 4};
@@ -214,7 +214,7 @@ static constexpr PlanSize kLargePlan{1, ~0ull};
 // 98; 24 vector programs x 100k 61 -> 37, 256 x 16,000 120 -> 80; 64 matrix
 // programs x 100k 140 -> 87; x 262,144 points: 4 vector programs 51 -> 27, 4 scalar
 // 49 -> 33, 8 matrix 90 -> 50, 4 2x2 matrix 90 -> 46 and 64 of them 377 -> 290.  At
-// 4096 vector programs x 100k one program an item is 20% slower.
+// 4096 vector programs x 100k one program an item takes 2.84 ms, four 2.30.
 // F+V3 with data sets of one and a half chunks an SM or more (on average over
 // the plan) keeps the full G: a group of G programs fills the device by itself, and
 // shares the features it reads.  On 1M points 4 vector programs take 73 us at 4
@@ -354,7 +354,7 @@ static void sort_by_key(std::vector<std::pair<uint64_t, uint32_t>> *v, std::vect
 // SM the spill depths share a launch, and up to one item on every other SM the
 // handler sets do too.  1024 scalar programs x 400 points, resident: 74 us as
 // three launches with a counter reset and a finalize launch, 55 us as one
-// launch without them.  Not where the deepest program's stacks would cost the others points
+// launch without them (32 us with one program an item since).  Not where the deepest program's stacks would cost the others points
 // per lane (end_plan halves P until a block fits) or the datasets' sizes ask
 // for different ones, so that no program's result depends on it.
 static void merge_small_launches(rsr_ctx *ctx, const Plan &plan, EncodeScratch *S, uint32_t n, PlanSize size, std::mutex *table_mu) {

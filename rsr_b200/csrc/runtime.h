@@ -241,7 +241,7 @@ struct rsr_ctx {
     rsr::TuneChoice force;     // set while the autotuner measures a candidate
     rsr::DevicePlan scratch;   // for one-shot calls
     rsr::DevicePlan pipe[2];   // one-shot calls split into chunks, alternating
-    rsr::HostBuf results;      // pinned results of a chunked one-shot call
+    rsr::HostBuf results;      // pinned results of the call at hand (a chunked one, or fetch_results)
     // Kept between calls so that encoding and planning a population of a
     // size seen before allocates nothing new: one encoding per program of
     // the largest population (or chunks, which alternate) so far, the host

@@ -74,7 +74,8 @@ enum AccBin : int { BIN_ADD = 0, BIN_SUB, BIN_RSUB, BIN_MUL, BIN_DIV, BIN_RDIV, 
 enum AccKind : int {
     K_F = 0, K_F_LDX = 0, K_F_LDC = 1, K_F_PUSH = 2, K_F_BIN = 3, K_F_UN = 21, K_F_END = 27,
     K_V2 = 32, K_V3 = 64, K_M2 = 104, K_M3 = 136, K_END = 163,
-    K_STOP = 31,  // ends a program (put behind its last word when it is staged)
+    K_STOP = 31,  // ends a program: behind its last word in the register kernel's code, behind each
+                  // sweep where the adjoint kernel stages it
     // offsets within the V2 / V3 blocks
     KV_LDX = 0, KV_LDC = 1, KV_PUSH = 2, KV_BIN = 3,
     // offsets within the M blocks

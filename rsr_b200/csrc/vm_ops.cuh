@@ -104,10 +104,10 @@ template <int P> __device__ __forceinline__ Vf<P> operator+(const Vf<P> &a, cons
 template <int P> __device__ __forceinline__ Vf<P> operator-(const Vf<P> &a, const Vf<P> &b) { Vf<P> r; RSR_LOOP r.v[k] = a.v[k] - b.v[k]; return r; }
 
 // Two points in one instruction (sm_100a's f32x2 forms; each half rounds like
-// the scalar one).  The assembler contracts a packed product with the packed
-// add or subtract it feeds, in spite of -fmad=false and .rn, so products are
+// the scalar one).  A packed product and the packed add or subtract it feeds
+// came out rounded once, in spite of -fmad=false and .rn, so products are
 // packed and the sums of products (operator+ and -) are not: no kernel may
-// hand a product to add2/sub2.  Packed sums are for a micro-op's own operands,
+// hand a product to add2/sub2 (tests/test_packed_ops.py).  Packed sums are for a micro-op's own operands,
 // which come from memory or from an earlier micro-op.  The interpreters are
 // bound by the instructions they issue, and this halves a micro-op's arithmetic:
 // 256 matrix programs x 1M points 2.18 -> 2.09 ms, gradients of 4096 vector
