@@ -34,9 +34,10 @@
 namespace rsr {
 
 constexpr uint32_t kAdjParams = 32;
-// Words of staged code beside the program's own: a stop entry (two words)
-// behind each sweep, and the entry read (not run) past the last one.
-constexpr uint32_t kAdjStopWords = 6;
+// Words of staged code beyond the program's own: a stop entry (two words)
+// behind each sweep, while the header is not staged.  The entry read (not run)
+// past the last one lies in the constants.
+constexpr uint32_t kAdjStopWords = 4 - kAdjHeaderWords;
 
 // The tape lives in tensor memory (tmem.cuh): one block per SM allocates
 // all 512 columns of its SM's 128 lanes; warp w owns lanes 32 (w % 4) ..
@@ -90,22 +91,22 @@ struct RevIO : AccIO<P> {
     }
     // Adds the lane's counted points of g, in order, to the sum of flat
     // parameter k (points past the dataset's end may carry 0*inf = NaN
-    // adjoints); parameters from kAdjParams on share a row nobody reads.  The
+    // adjoints); the sums of parameters from kAdjParams on are not stored.  The
     // branch is on the tile being cut off, which is so for the whole warp.
     // One asm statement, so that nvcc has no branch here to keep the adjoints
     // apart for: gradients of 4096 vector programs x 100k points 10.99 ms with
     // the sum as a loop in C++, 10.67 so (256 matrix programs x 1M points 8.75
     // and 8.76).
     __device__ __forceinline__ void grad_add(uint32_t k, const Vf<P> &g) const {
-        const uint32_t row = gacc + 128u * min(k, kAdjParams);
+        const uint32_t row = gacc + 128u * min(k, kAdjParams - 1u);
         if constexpr (P == 2) {
-            asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\n"
+            asm volatile("{\n.reg .pred p, q;\n.reg .b32 b;\n.reg .f32 s, o;\n"
                          "and.b32 b, %3, 1;\nsetp.ne.u32 p, b, 0;\nmov.f32 s, 0f00000000;\n@p add.rn.f32 s, s, %1;\n"
                          "and.b32 b, %3, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
-                         "ld.shared.f32 o, [%0];\nadd.rn.f32 o, o, s;\nst.shared.f32 [%0], o;\n}"
-                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "r"(valid) : "memory");
+                         "ld.shared.f32 o, [%0];\nadd.rn.f32 o, o, s;\nsetp.lt.u32 q, %4, %5;\n@q st.shared.f32 [%0], o;\n}"
+                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "r"(valid), "r"(k), "n"(kAdjParams) : "memory");
         } else if constexpr (P == 4) {
-            asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
+            asm volatile("{\n.reg .pred p, q;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
                          "mov.f32 s, 0f00000000;\nsetp.gt.u32 p, %5, 15;\n@p bra.uni PART;\n"
                          "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\nbra.uni DONE;\n"
                          "PART:\n"
@@ -113,10 +114,10 @@ struct RevIO : AccIO<P> {
                          "and.b32 b, %5, 2;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %2;\n"
                          "and.b32 b, %5, 4;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %3;\n"
                          "and.b32 b, %5, 8;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %4;\n"
-                         "DONE:\nadd.rn.f32 o, o, s;\nst.shared.f32 [%0], o;\n}"
-                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "r"(valid) : "memory");
+                         "DONE:\nadd.rn.f32 o, o, s;\nsetp.lt.u32 q, %6, %7;\n@q st.shared.f32 [%0], o;\n}"
+                         ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "r"(valid), "r"(k), "n"(kAdjParams) : "memory");
         } else {
-            asm volatile("{\n.reg .pred p;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
+            asm volatile("{\n.reg .pred p, q;\n.reg .b32 b;\n.reg .f32 s, o;\nld.shared.f32 o, [%0];\n"
                          "mov.f32 s, 0f00000000;\nsetp.gt.u32 p, %9, 255;\n@p bra.uni PART;\n"
                          "add.rn.f32 s, s, %1;\nadd.rn.f32 s, s, %2;\nadd.rn.f32 s, s, %3;\nadd.rn.f32 s, s, %4;\n"
                          "add.rn.f32 s, s, %5;\nadd.rn.f32 s, s, %6;\nadd.rn.f32 s, s, %7;\nadd.rn.f32 s, s, %8;\nbra.uni DONE;\n"
@@ -129,9 +130,9 @@ struct RevIO : AccIO<P> {
                          "and.b32 b, %9, 32;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %6;\n"
                          "and.b32 b, %9, 64;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %7;\n"
                          "and.b32 b, %9, 128;\nsetp.ne.u32 p, b, 0;\n@p add.rn.f32 s, s, %8;\n"
-                         "DONE:\nadd.rn.f32 o, o, s;\nst.shared.f32 [%0], o;\n}"
+                         "DONE:\nadd.rn.f32 o, o, s;\nsetp.lt.u32 q, %10, %11;\n@q st.shared.f32 [%0], o;\n}"
                          ::"r"(row), "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "f"(g.v[4]), "f"(g.v[5]),
-                         "f"(g.v[6]), "f"(g.v[7]), "r"(valid) : "memory");
+                         "f"(g.v[6]), "f"(g.v[7]), "r"(valid), "r"(k), "n"(kAdjParams) : "memory");
         }
     }
 };
@@ -677,14 +678,15 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
             io.gacc = opaque(at + 4u * lane - 4u * lane_point<P>(lane, 0));
         }
         const uint32_t np = min(pd.n_consts, kAdjParams);
-        const uint32_t sse = io.gacc + 4u * lane + (np + (pd.n_consts > kAdjParams)) * 128u;  // this lane's squared errors (f64, a row of 256 bytes)
+        const uint32_t sse = io.gacc + 4u * lane + np * 128u;  // this lane's squared errors (f64, a row of 256 bytes)
         const uint32_t *gcode = a.code + pd.uop_off;
-        // the code, with a stop entry behind each sweep
-        const uint32_t cut = kAdjHeaderWords + 2u * __ldg(gcode);
-        for (uint32_t i = threadIdx.x; i < pd.uop_len; i += blockDim.x) scode[i < cut ? i : i + 2u] = __ldg(gcode + i);
+        // the two sweeps' entries, with a stop entry behind each
+        const uint32_t cut = 2u * __ldg(gcode), n_code = pd.uop_len - kAdjHeaderWords;
+        for (uint32_t i = threadIdx.x; i < n_code; i += blockDim.x)
+            scode[i < cut ? i : i + 2u] = __ldg(gcode + kAdjHeaderWords + i);
         const DatasetDesc ds = a.datasets[pd.dataset];
         if (threadIdx.x == 0) {
-            scode[cut] = scode[pd.uop_len + 2u] = K_STOP;
+            scode[cut] = scode[n_code + 2u] = K_STOP;
             *reinterpret_cast<int64_t *>(meta + 2) =
                 reinterpret_cast<const char *>(ds.y) - reinterpret_cast<const char *>(ds.x);
         }
@@ -693,7 +695,7 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
         sts_f64(sse, 0.0);
         __syncthreads();
         io.stride = opaque((uint32_t)ds.stride);
-        const uint32_t fwd = opaque(smem_addr(scode + kAdjHeaderWords)), rev = opaque(smem_addr(scode + cut + 2u));
+        const uint32_t fwd = opaque(smem_addr(scode)), rev = opaque(smem_addr(scode + cut + 2u));
         // The item's parts (kPartPoints points each) one after another; a
         // warp takes the same tiles of a part, and sums them the same way,
         // whatever the item's size, so a program's partial sums do not
@@ -796,15 +798,14 @@ __global__ void __launch_bounds__(adj_warps<PROF, P>() * 32, 1) adj_eval_kernel(
 // Shared-memory layout (floats).  Block header: code (+ stop entries) | constants |
 // meta (4 words) | cross-warp sums (parts x warps x 33 doubles).  Per warp: stacks
 // (per type; the reverse sweep's adjoint stacks in the same slots) |
-// gradient sums (one row of 32 per parameter, at most 32, and one for all
-// parameters past them) | squared errors (a
+// gradient sums (one row of 32 per parameter, at most 32) | squared errors (a
 // row of 32 doubles), each program's own sizes (the kernel lays the region out per item);
 // warp_floats is the largest region of the launch.  The tape is in tensor
 // memory (a.tmem_cols columns a warp).
 uint32_t adj_warp_floats(const uint32_t *stack_depth, int P, uint32_t n_params) {
     uint32_t slots = 0;  // the stacks, whose slots the adjoints reuse
     for (int t = 0; t < N_STACKS; ++t) slots += stack_depth[t] * (uint32_t)kStackWidth[t];
-    const uint32_t np = n_params <= kAdjParams ? n_params : kAdjParams + 1;
+    const uint32_t np = n_params < kAdjParams ? n_params : kAdjParams;
     return (slots * 32u * (uint32_t)P + np * 32u + 2u * 32u + 3u) & ~3u;
 }
 
