@@ -120,14 +120,16 @@ constexpr uint32_t kEnd = 0xFFFFFFFFu;       // no program at this address
 // What a block keeps of its work item in shared memory (words).
 enum RegMeta : uint32_t {
     M_PROGS = 0,       // [g][2] shared-memory addresses of each program's code and constants, kEnd behind the last
-    M_PROLOGUES = 18,  // [g] address of its prologue, kEnd if it has none
-    M_Y_OFF = 26,      // targets' byte distance from the features
-    M_N_EVAL = 28,     // points to count
-    M_ITEM = 30, M_FULL_TILES, M_TILE_BEGIN, M_TILE_END, M_PROG_BEGIN, M_HOISTED,
-    kMetaWords = 36
+    M_Y_OFF = 18,      // targets' byte distance from the features
+    M_N_EVAL = 20,     // points to count
+    M_ITEM = 22, M_FULL_TILES, M_TILE_BEGIN, M_TILE_END, M_PROG_BEGIN, M_HOISTED,
+    kMetaWords = 32,
+    // [g] address of its prologue, kEnd if it has none: in the room of the
+    // cross-warp sums, which are written when every prologue has run
+    M_PROLOGUES = kMetaWords
 };
-static_assert(M_PROLOGUES == M_PROGS + 2 * (kMaxProgsPerWarp + 1) && M_Y_OFF == M_PROLOGUES + kMaxProgsPerWarp &&
-              M_HOISTED + 1 == kMetaWords && kMetaWords % 4 == 0, "RegMeta layout");
+static_assert(M_Y_OFF == M_PROGS + 2 * (kMaxProgsPerWarp + 1) && M_HOISTED < kMetaWords && kMetaWords % 4 == 0,
+              "RegMeta layout");
 
 // Block-cooperative item loop.  All warps of a block run the same programs
 // (one work item) on different tiles of the item's chunk, so the SM's
