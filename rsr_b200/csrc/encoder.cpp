@@ -1088,6 +1088,7 @@ int encode_program(const uint32_t *code, uint32_t len, const uint8_t *kinds, uin
             n_hoist = 0;
         }
         if (!hoist.empty()) {
+            E.hoists = true;
             for (size_t i = 0; i < nodes.size(); ++i)
                 if (live[i] && nodes[i].is_const) hoisted_flops += op_sig(nodes[i].opcode).flops;
             AccEmitter em(nodes);

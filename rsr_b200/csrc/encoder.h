@@ -46,6 +46,7 @@ struct EncodedProgram {
     uint32_t main_off = 0;                // first word of the main program (FORM_HOIST: behind the prologue)
     uint32_t n_hoist = 0;                 // floats the prologue adds to the constants
     uint32_t hoisted_flops = 0;           // operations of flops_per_point that the prologue runs once an item
+    bool hoists = false;                  // FORM_HOIST found constant subtrees
     // adjoint (slot form with one slot range per value, never reused)
     std::vector<uint32_t> tape_code;      // 2 header words + 5 words per live node
     uint32_t n_tape_val = 0, n_tape_adj = 0;  // scalar value / adjoint slots

@@ -491,6 +491,10 @@ static int begin_plan(rsr_ctx *ctx, const rsr_population &pop, const uint64_t *d
         };
         if (!encode(forms)) return;
         int path = forms & FORM_ADJ ? adjoint_path(E, &S->adj_omit[i]) : forms & FORM_ACC ? register_path(E) : -1;
+        if (path < 0 && E.hoists) {  // too long or too deep with a prologue: perhaps not without
+            if (!encode(FORM_ACC)) return;
+            path = register_path(E);
+        }
         if (gradient && path < 0) {
             if (!(forms & FORM_TAPE) && !encode(FORM_TAPE)) return;
             path = slot_adjoint_path(E);

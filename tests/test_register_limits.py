@@ -47,6 +47,29 @@ def test_block_size(per_item):
             assert g["smem_bytes"] == _bytes(words[i] * per_item, p.param_count() * per_item, stack, per_item), i
 
 
+def _with_prologue(n):
+    """c_0 * c_1 + x + .. + x: as accumulator code n + 2 words, hoisted 3 more."""
+    code = [I.load_const(FLOAT, 0), I.load_const(FLOAT, 1), I.op("MulF")] + [I.load_var(FLOAT, 0), I.op("AddF")] * n
+    return Program(code, [Scalar(FLOAT, (1.5,)), Scalar(FLOAT, (2.0,))])
+
+
+def test_a_prologue_does_not_push_a_program_off_the_kernel():
+    """The longest program that fits without its constant subtree hoisted: it runs that way."""
+    n = next(n for n in range(24_900, 25_000) if _bytes(n + 4, 2, 0, 1) > 100 * 1024)
+    longest = _with_prologue(n)
+    plain, hoisted = (len(E.encoding(longest, 1, 1)), len(E.encoding(longest, 1, 6)) - 3)
+    assert (plain, hoisted) == (n + 2, n + 5)
+    assert _bytes(plain + 1, 2, 0, 1) <= 100 * 1024 < _bytes(hoisted + 1, 3, 0, 1)
+    with E.Engine() as e:
+        d = e.upload(Dataset.new(np.zeros((8, 1), f32), np.zeros(8, f32), [FLOAT]))
+        mse, (g,) = _run(e, [longest], d)
+        assert g["kernel"] == "register" and mse[0] == 9.0
+        assert e.compute_mse(longest, d) == 9.0
+        short = _with_prologue(10)
+        mse, groups = _run(e, [longest, short, longest, short], d)
+        assert (mse == 9.0).all() and {g["kernel"] for g in groups} == {"register"}
+
+
 def test_prologues_and_sums_share_their_room():
     """Eight programs an item, all with prologues, over items of many tiles: the sums of one item are
     taken where its prologues' addresses stood, and the next item's addresses are laid there again."""
