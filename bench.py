@@ -53,10 +53,10 @@ sys.path.insert(0, str(ROOT))
 # this workload (three spill-depth classes, P=8 G=4), from one ncu capture of
 # `bench.py --case --workload vector --programs 4096 --kernel register --runs 3
 # --points-per-thread 8 --programs-per-warp 4` (dram__bytes_read/write.sum):
-# 4,711,424 + 4,775,680 + 4,116,736 read, 512 written.  ncu replays each launch
+# 4,468,224 + 4,966,656 + 4,105,472 read, none written.  ncu replays each launch
 # with cold caches, so each re-reads the 4 MB dataset; in a step the second
 # and third launches find it in L2.
-DOMINANT_KERNEL_DRAM_BYTES = 13_604_352
+DOMINANT_KERNEL_DRAM_BYTES = 13_540_352
 METRIC = "program_points_per_sec"
 UNIT = "program*points/s"
 N_PROGRAMS = 4096
